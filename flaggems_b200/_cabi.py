@@ -1,9 +1,12 @@
-"""ctypes binding of the C-ABI library (include/flaggems_b200.h).
+"""Bindings of the C-ABI library (include/flaggems_b200.h): ctypes for every entry point, and the
+native host module (csrc/host.cpp) that takes the ordinary calls without the interpreter's overhead.
 
 The library is the only compute path: if it is missing or an entry point fails,
 the caller gets an exception; there is no fallback of any kind.
 """
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 from ctypes import c_char_p, c_float, c_int, c_int32, c_int64, c_uint, c_uint64, c_void_p
 
@@ -11,6 +14,7 @@ import torch
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "lib", "libflaggems_b200.so")
+HOST_PATH = os.path.join(_HERE, "lib", "_fg_host.so")
 
 FG_OK = 0
 DTYPE_CODE = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
@@ -127,6 +131,23 @@ def lib():
             fn.argtypes = args
         _lib = handle
     return _lib
+
+
+class _NativeHost:
+    """The functions of the native host module, loaded at the first use (raises when it is absent).
+    Each returns None for a call that it leaves to the Python code behind it."""
+
+    def __getattr__(self, name):
+        if not os.path.exists(HOST_PATH):
+            raise FlagGemsB200Error(f"{HOST_PATH} not found: build it with `python -m flaggems_b200.build`.")
+        loader = importlib.machinery.ExtensionFileLoader("_fg_host", HOST_PATH)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_fg_host", loader))
+        loader.exec_module(module)
+        self.__dict__.update({k: v for k, v in vars(module).items() if not k.startswith("_")})
+        return self.__dict__[name]
+
+
+host = _NativeHost()
 
 
 def check(rc):

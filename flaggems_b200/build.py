@@ -1,9 +1,9 @@
-"""Build the C-ABI shared library with nvcc for sm_100a.
+"""Build the C-ABI shared library with nvcc for sm_100a, and the native host module over it.
 
     python -m flaggems_b200.build [--force] [--verbose]
 
-Produces ``flaggems_b200/lib/libflaggems_b200.so`` next to the sources (in-tree,
-git-ignored).  nvcc cross-compiles without a GPU.  No fast-math flags: the
+Produces ``flaggems_b200/lib/libflaggems_b200.so`` and ``lib/_fg_host.so`` next to the sources
+(in-tree, git-ignored).  nvcc cross-compiles without a GPU.  No fast-math flags: the
 quantisation kernels rely on IEEE fp32 semantics.
 """
 import argparse
@@ -11,11 +11,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libflaggems_b200.so")
+HOST_PATH = os.path.join(LIB_DIR, "_fg_host.so")
 SOURCES = ["api.cu", "quant.cu", "moe_glue.cu", "moe_layer.cu", "router.cu", "gemm_fp8_sm100.cu"]
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
@@ -27,18 +29,41 @@ def _nvcc():
     return cand
 
 
-def _stale():
-    if not os.path.exists(LIB_PATH):
+def _stale(path, sources):
+    if not os.path.exists(path):
         return True
-    t = os.path.getmtime(LIB_PATH)
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
+    deps = [os.path.join(CSRC, f) for f in sources]
     deps.append(os.path.join(os.path.dirname(HERE), "include", "flaggems_b200.h"))
-    return any(os.path.getmtime(d) > t for d in deps)
+    return any(os.path.getmtime(d) > os.path.getmtime(path) for d in deps)
 
 
 def build(force=False, verbose=False):
-    if not force and not _stale():
-        return LIB_PATH
+    if force or _stale(LIB_PATH, [f for f in os.listdir(CSRC) if f != "host.cpp"]):
+        build_library(verbose)
+    if force or _stale(HOST_PATH, ["host.cpp"]):
+        build_host()
+    return LIB_PATH
+
+
+def build_host():
+    """The CPython module over the library, against the headers of the installed torch."""
+    import torch
+
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    cxx = os.environ.get("CXX") or shutil.which("g++") or "c++"
+    cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f"-I{os.path.join(root, 'include')}", f"-I{os.path.join(root, 'include', 'torch', 'csrc', 'api', 'include')}",
+           f"-I{os.path.join(cuda, 'include')}", f"-I{sysconfig.get_paths()['include']}",
+           os.path.join(CSRC, "host.cpp"), "-o", HOST_PATH, f"-L{os.path.join(root, 'lib')}",
+           "-ltorch", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10", "-lc10_cuda",
+           f"-L{LIB_DIR}", "-lflaggems_b200", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("the native host module failed to build:\n" + r.stdout)
+
+
+def build_library(verbose=False):
     os.makedirs(LIB_DIR, exist_ok=True)
     objs = []
     procs = []
@@ -65,7 +90,6 @@ def build(force=False, verbose=False):
     r = subprocess.run(link, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if r.returncode != 0:
         raise RuntimeError("link failed:\n" + r.stdout)
-    return LIB_PATH
 
 
 if __name__ == "__main__":

@@ -25,6 +25,10 @@ def act_quant_triton(
     no Triton is involved.)
     """
     logger.debug("GEMS ACT_QUANT")
+    if x.is_cuda:
+        done = _cabi.host.act_quant(x, block_size, scale_fmt is not None)
+        if done is not None:
+            return done
     assert x.is_contiguous(), "Input tensor must be contiguous"
     assert (
         x.size(-1) % block_size == 0

@@ -171,6 +171,15 @@ def _fp8_quantize(A, A_scale, per_act_token, block_shape=None):
     """FP8 e4m3 quantisation of MoE activations: block-wise, per-token, or per-tensor with a
     given or a dynamic scale (reference: fused_moe.py:629-698)."""
     _cabi.require_cuda(A)
+    if block_shape is None:
+        if per_act_token:
+            done = _cabi.host.token_quant(A)
+            if done is not None:
+                return done
+        elif A_scale is not None:
+            q = _cabi.host.tensor_quant(A, A_scale)
+            if q is not None:
+                return q, A_scale
     with _cabi.device_guard(A):
         if block_shape is not None:
             assert not per_act_token

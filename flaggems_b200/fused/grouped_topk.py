@@ -28,6 +28,11 @@ def grouped_topk(
     """``expert_counts`` (int32 [num_experts], optional, not in the reference) receives the number
     of route slots per expert added to its current content."""
     logger.debug("GEMS GROUPED TOPK")
+    if scores.is_cuda and expert_counts is None:
+        done = _cabi.host.grouped_topk(scores, n_group, topk_group, topk, renormalize, float(routed_scaling_factor), bias,
+                                       scoring_func)
+        if done is not None:
+            return done
     if scores.ndim != 2:
         raise ValueError("scores must be a 2D Tensor")
     num_tokens, num_experts = scores.shape

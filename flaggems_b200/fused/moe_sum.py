@@ -13,6 +13,8 @@ logger = logging.getLogger(__name__.replace("flaggems_b200", "flag_gems", 1))
 
 def moe_sum(input: torch.Tensor, output: torch.Tensor):
     logger.debug("GEMS MOE SUM")
+    if input.is_cuda and _cabi.host.moe_sum(input, output) is not None:
+        return output
     assert input.dim() == 3 and output.dim() == 2, "input must be [M, topk, K] and output [M, K]"
     m, topk, k = input.shape
     assert output.shape == (m, k), "output shape mismatch"

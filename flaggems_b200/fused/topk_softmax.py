@@ -26,6 +26,9 @@ def topk_softmax(
     """``expert_counts`` (int32 [num_experts], optional, not in the reference) receives the number
     of route slots per expert added to its current content."""
     logger.debug("GEMS TOPK SOFTMAX")
+    if gating_output.is_cuda and expert_counts is None:
+        if _cabi.host.topk_softmax(topk_weights, topk_indices, token_expert_indices, gating_output, renormalize):
+            return
     num_tokens, num_experts = gating_output.shape
     topk = topk_weights.size(-1)
     assert topk <= 32

@@ -24,6 +24,10 @@ def per_token_group_quant_fp8(
 ) -> Tuple[torch.Tensor, torch.Tensor]:
     logger.debug("GEMS PER TOKEN GROUP QUANT FP8")
     fp8_dtype = SUPPORTED_FP8_DTYPE if dtype is None else dtype
+    if x.is_cuda and fp8_dtype is SUPPORTED_FP8_DTYPE:
+        done = _cabi.host.group_quant(x, group_size, eps, column_major_scales, scale_ue8m0)
+        if done is not None:
+            return done
     assert x.shape[-1] % group_size == 0, (
         f"the last dimension of `x` {x.shape[-1]} must be divisible "
         f"by `group_size` {group_size}"

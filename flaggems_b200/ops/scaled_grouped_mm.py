@@ -148,6 +148,10 @@ def _grouped_rows(a, w_gnk, scale_a, scale_b, offs, bias, out_dtype):
 def scaled_grouped_mm(self, mat2, scale_a, scale_b, offs=None, bias=None, scale_result=None, out_dtype=None,
                       use_fast_accum=False):
     logger.debug("GEMS SCALED_GROUPED_MM")
+    if self.is_cuda and bias is None and scale_result is None and offs is not None:
+        out = _cabi.host.grouped_mm(self, mat2, scale_a, scale_b, offs, out_dtype or _default_out_dtype(self.dtype))
+        if out is not None:
+            return out
     if scale_result is not None:
         raise RuntimeError("scale_result is not supported for scaled_grouped_mm")
     _check_dims(self, mat2)

@@ -116,10 +116,17 @@ def _scaled_mm_impl(self, mat2, scale_a, scale_b, bias, out_dtype, out):
 
 def scaled_mm(self, mat2, scale_a, scale_b, bias=None, scale_result=None, out_dtype=None, use_fast_accum=False):
     logger.debug("GEMS SCALED_MM")
+    if self.is_cuda:
+        out = _cabi.host.scaled_mm_new(self, mat2, scale_a, scale_b, bias, self.dtype if out_dtype is None else out_dtype)
+        if out is not None:
+            return out
     return _scaled_mm_impl(self, mat2, scale_a, scale_b, bias, out_dtype, None)
 
 
 def scaled_mm_out(self, mat2, scale_a, scale_b, bias=None, scale_result=None, out_dtype=None,
                   use_fast_accum=False, *, out):
     logger.debug("GEMS SCALED_MM_OUT")
+    if self.is_cuda and (out_dtype is None or out.dtype == out_dtype):
+        if _cabi.host.scaled_mm(out, self, mat2, scale_a, scale_b, bias, False) is not None:
+            return out
     return _scaled_mm_impl(self, mat2, scale_a, scale_b, bias, out_dtype, out)

@@ -25,6 +25,10 @@ def w8a8_block_fp8_matmul(
     output_dtype: torch.dtype = torch.bfloat16,
 ) -> torch.Tensor:
     logger.debug("GEMS W8A8_BLOCK_FP8_MATMUL")
+    if A.is_cuda:
+        c = _cabi.host.block_mm(A, B, As, Bs, block_size, output_dtype)
+        if c is not None:
+            return c
     assert len(block_size) == 2
     block_n, block_k = block_size[0], block_size[1]
     assert A.shape[-1] == B.shape[-1]
