@@ -109,7 +109,8 @@ struct GemmParams {
 // In block-scaled mode those warps are needed in every K block, so whatever they do at a tile's end
 // stalls the tensor core once its two accumulator buffers are full.  The parked tile takes the
 // room of one ring stage (three stages instead of four).
-template <int BN, bool SMALL_A, bool PAIR = false, bool ASTORE = false>
+// COLVEC (plain epilogue, no split-K): room for a tile's column scales and bias in shared memory.
+template <int BN, bool SMALL_A, bool PAIR = false, bool ASTORE = false, bool COLVEC = false>
 struct Cfg {
     static_assert(!ASTORE || (BN == 256 && !SMALL_A && !PAIR), "the store warp serves the 256-wide tile");
     static_assert(BN == 32 || BN == 64 || BN == 128 || BN == 256, "unsupported tile width");
@@ -140,8 +141,9 @@ struct Cfg {
     static constexpr int BAR_BYTES = 512;  // (2*STAGES + 6) mbarriers, TMEM base slot, abort flag, turn counter
     static_assert((2 * STAGES + 6) * 8 + 16 <= BAR_BYTES, "barrier area too small");
     static constexpr int EPI_STAGE_BYTES = 2048;  // per epilogue warp: 32 rows x 64 bytes
-    static constexpr int SMEM_BYTES =
-        STAGES * STAGE_BYTES + TAIL_PAD + BAR_BYTES + EPI_WARPS * EPI_STAGE_BYTES + PARK_BYTES + 1024;
+    static constexpr int COL_BYTES = COLVEC ? 2 * COLS * 4 : 0;  // per epilogue warp: its columns' scales, then bias
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + TAIL_PAD + BAR_BYTES +
+                                      EPI_WARPS * (EPI_STAGE_BYTES + COL_BYTES) + PARK_BYTES + 1024;
     static_assert(SMEM_BYTES <= 232448, "over the 227 KB shared memory limit");
     // split-K parks a 128 x BN fp32 partial tile (rows padded by 4 floats) in the ring's memory
     static_assert(SMALL_A || PAIR || BLOCK_M * (BN + 4) * 4 <= STAGES * STAGE_BYTES, "partial tile does not fit");
@@ -296,7 +298,7 @@ template <int BN, bool BLOCK_SCALED, bool FUSE_SILU, bool SMALL_A, bool SPLITK, 
 __global__ void __launch_bounds__(Cfg<BN, SMALL_A, PAIR, ASTORE>::THREADS, 1)
 gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                 const GemmParams p) {
-    using C = Cfg<BN, SMALL_A, PAIR, ASTORE>;
+    using C = Cfg<BN, SMALL_A, PAIR, ASTORE, !BLOCK_SCALED && !SPLITK>;
     static_assert(!ASTORE || (BLOCK_SCALED && !SPLITK), "the store warp serves the block-scaled tiles");
     constexpr bool INT8 = OPK == 1;
     static_assert(OPK == 0 || (!BLOCK_SCALED && !SPLITK && !PAIR && !SMALL_A), "int8 and 16-bit operands serve the plain and grouped tiles");
@@ -730,11 +732,34 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
 
             if constexpr (!BLOCK_SCALED) {
                 const uint32_t buf = acc_iter & 1u;
+                // The tile's column scales and bias are fetched while its MMAs run, one coalesced load per
+                // 32 columns, and read back from shared memory as broadcasts.  Loading them per element
+                // cost a global-memory latency per column of a tile (40 us of the 58 us of a single-wave
+                // product such as 16 x 28672 x 4096).
+                const float sa = p.sa_mode == FG_SCALE_VECTOR ? p.sa[srow] : p.sa[0];
+                float* col_scale = reinterpret_cast<float*>(epi_stage_base + C::EPI_WARPS * C::EPI_STAGE_BYTES + ew * C::COL_BYTES);
+                float* col_bias = col_scale + C::COLS;
+                if constexpr (!SPLITK) {
+                    const float* sbp = p.sb + (p.sb_mode == FG_SCALE_VECTOR ? (int64_t)expert * p.sb_stride_e : (int64_t)expert * (p.grouped ? 1 : 0));
+                    float s[C::COLS / 32], b[C::COLS / 32];
+#pragma unroll
+                    for (int c = 0; c < C::COLS / 32; ++c) {
+                        const int n = min(out_col_base + 32 * (FUSE_SILU ? (c & 1) : c) + lane, p.n_out - 1);
+                        const int up = FUSE_SILU && c >= 2 ? p.N / 2 : 0;
+                        s[c] = p.sb_mode == FG_SCALE_VECTOR ? __ldg(sbp + up + n) : __ldg(sbp);
+                        b[c] = p.bias ? load_as_float(p.bias, p.bias_dtype, n + (int64_t)expert * p.bias_stride_e) : 0.0f;
+                    }
+                    __syncwarp();  // every lane has read the previous tile's values
+#pragma unroll
+                    for (int c = 0; c < C::COLS / 32; ++c) {
+                        col_scale[32 * c + lane] = s[c];
+                        col_bias[32 * c + lane] = b[c];
+                    }
+                    __syncwarp();
+                }
                 ok = mbar_wait(&tmem_full[buf], (acc_iter >> 1) & 1u, abort_flag, p.status, 4);
                 if (!ok) break;
                 tc_fence_after_sync();
-                const float sa = p.sa_mode == FG_SCALE_VECTOR ? p.sa[srow] : p.sa[0];
-                const float* sbp = p.sb + (p.sb_mode == FG_SCALE_VECTOR ? (int64_t)expert * p.sb_stride_e : (int64_t)expert * (p.grouped ? 1 : 0));
                 const uint32_t tbuf = lane_addr + buf * BN;
 #pragma unroll
                 for (int c = 0; c < OUT_CHUNKS; ++c) {
@@ -746,14 +771,10 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                         tmem_ld_32x32b_x32(tbuf + 64 * half + 32 * c, raw);
                         tmem_ld_32x32b_x32(tbuf + BN / 2 + 64 * half + 32 * c, raw_up);
                         tmem_ld_wait();
-                        const int up_off = p.N / 2;
 #pragma unroll
                         for (int i = 0; i < 32; ++i) {
-                            const int n = min(col + i, p.n_out - 1);
-                            const float sg = p.sb_mode == FG_SCALE_VECTOR ? __ldg(sbp + n) : sbp[0];
-                            const float su = p.sb_mode == FG_SCALE_VECTOR ? __ldg(sbp + up_off + n) : sbp[0];
-                            const float g = acc_f(raw[i]) * sa * sg;
-                            const float u = acc_f(raw_up[i]) * sa * su;
+                            const float g = acc_f(raw[i]) * sa * col_scale[32 * c + i];
+                            const float u = acc_f(raw_up[i]) * sa * col_scale[64 + 32 * c + i];
                             v[i] = silu_mul(g, u);
                         }
                     } else if constexpr (SPLITK) {
@@ -767,16 +788,13 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                         tmem_ld_32x32b_x32(tbuf + 128 * half + 32 * c, raw);
                         tmem_ld_wait();
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) {
-                            const int n = min(col + i, p.n_out - 1);
-                            const float sb = p.sb_mode == FG_SCALE_VECTOR ? __ldg(sbp + n) : sbp[0];
-                            float x = sb * (sa * acc_f(raw[i]));
-                            x *= weight;
-                            if (p.bias) {
-                                const float b = load_as_float(p.bias, p.bias_dtype, n + (int64_t)expert * p.bias_stride_e);
-                                x = p.bias_after_round ? round_through(x, p.out_dtype) + b : x + b;
+                        for (int i = 0; i < 32; ++i) v[i] = col_scale[32 * c + i] * (sa * acc_f(raw[i])) * weight;
+                        if (p.bias) {
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) {
+                                const float b = col_bias[32 * c + i];
+                                v[i] = p.bias_after_round ? round_through(v[i], p.out_dtype) + b : v[i] + b;
                             }
-                            v[i] = x;
                         }
                     }
                     if constexpr (!SPLITK) {
@@ -1200,7 +1218,7 @@ int launch_splitk(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams
 // trip MMA -> both CTAs' epilogues -> MMA through cluster-wide barriers, and that latency costs
 // more than the halved B traffic saves (measured: about half the single-CTA throughput).
 int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int pair_tiles, cudaStream_t st) {
-    using C = Cfg<256, false, true>;
+    using C = Cfg<256, false, true, false, true>;
     auto kernel = gemm_fp8_kernel<256, false, false, false, false, true>;
     static int max_clusters_dev[64];
     static std::mutex mu;
@@ -1246,7 +1264,7 @@ bool pair_enabled() {
 
 template <int BN, bool BS, bool SILU, bool SMALL_A = false, bool ASTORE = false, int OPK = 0>
 int launch_inst(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int max_tiles, cudaStream_t st) {
-    using C = Cfg<BN, SMALL_A, false, ASTORE>;
+    using C = Cfg<BN, SMALL_A, false, ASTORE, !BS>;
     auto kernel = gemm_fp8_kernel<BN, BS, SILU, SMALL_A, false, false, ASTORE, OPK>;
     static bool attr_done[64];
     static std::mutex mu;
