@@ -211,16 +211,13 @@ __global__ void __launch_bounds__(256) group_quant_kernel(QuantArgs a) {
     }
 }
 
-// ---- small groups, 16-bit inputs: the bandwidth path ---------------------------------------
-// A lane owns 16 consecutive elements (two 16-byte loads, one 16-byte store), a team of
-// GROUP/16 lanes owns a group.  The inputs stay in registers as raw 16-bit pairs: max|x| is taken
-// on the pairs (exact in the input type), and they are widened to fp32 only where they are
-// scaled, so that a thread carries 8 registers of data per group in flight instead of 16 and five
-// CTAs (40 warps, 48 registers each) fit an SM; six CTAs spill and measured no faster.  PACKED selects the expert-parallel dispatch format (scales and a trailer behind
-// the payload of each row, rows optionally stored into peers' receive buffers).
-template <typename T, int MODE, int TPG, bool PACKED>
-__global__ void __launch_bounds__(256, 5) group_quant16_kernel(QuantArgs a) {
-    constexpr int UNROLL = 2;
+// ---- the expert-parallel dispatch format, 16-bit inputs, groups of 128 -------------------------------
+// Scales and a trailer sit behind the payload of each row, and rows are optionally stored into peers'
+// receive buffers.  A lane owns 16 consecutive elements (two 16-byte loads, one 16-byte store), kept as
+// raw 16-bit pairs; a team of eight lanes owns a group.
+template <typename T, int MODE>
+__global__ void __launch_bounds__(256, 5) group_pack16_kernel(QuantArgs a) {
+    constexpr int UNROLL = 2, TPG = 8;
     constexpr int GROUP = TPG * 16;
     using P = Pair16<T>;
     const int64_t rows = resolve_rows(a);
@@ -267,7 +264,7 @@ __global__ void __launch_bounds__(256, 5) group_quant16_kernel(QuantArgs a) {
             const float s = make_scale<MODE>(amax, a.eps, a.pow2);
             const Divider d = make_divider<MODE>(s);
             uint8_t* qrow = nullptr;
-            if (row[u] < rows) qrow = PACKED ? packed_row_ptr(a, row[u]) : a.q + (int64_t)row[u] * a.ld_q;
+            if (row[u] < rows) qrow = packed_row_ptr(a, row[u]);
             if (qrow) {
                 uint32_t o[4];
 #pragma unroll
@@ -283,12 +280,8 @@ __global__ void __launch_bounds__(256, 5) group_quant16_kernel(QuantArgs a) {
                 }
                 *reinterpret_cast<uint4*>(qrow + cg[u] * GROUP + lane_in_team * 16) = make_uint4(o[0], o[1], o[2], o[3]);
                 if (lane_in_team == 0) {
-                    if constexpr (PACKED) {  // scales sit behind the payload of the same row
-                        reinterpret_cast<float*>(qrow + a.K)[cg[u]] = s;
-                        if (cg[u] == 0) write_row_meta(a, row[u]);
-                    } else {
-                        a.s[(int64_t)row[u] * a.s_row_stride + (int64_t)cg[u] * a.s_col_stride] = s;
-                    }
+                    reinterpret_cast<float*>(qrow + a.K)[cg[u]] = s;
+                    if (cg[u] == 0) write_row_meta(a, row[u]);
                 }
             }
             cg[u] += step_cg;
@@ -429,6 +422,70 @@ __global__ void __launch_bounds__(256) row_quant_kernel(QuantArgs a) {
 // copies of the row in registers ran at 2.9 TB/s (8192 x 14336: 123 us).
 constexpr int ROW_UNITS = 2;  // units of 16 elements per thread
 
+// Sixteen elements (two raw vectors) -> sixteen output bytes.
+template <typename T, int MODE, int DMODE>
+__device__ __forceinline__ uint4 quantize16(const uint4 (&v)[2], const Divider& d) {
+    uint2 o[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const uint32_t w[4] = {v[h].x, v[h].y, v[h].z, v[h].w};
+        float f[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float lo, hi;
+            Pair16<T>::widen(w[i], lo, hi);
+            apply_divider2<DMODE>(lo, hi, d, f[2 * i], f[2 * i + 1]);
+        }
+        o[h] = pack_out8<MODE>(f);
+    }
+    return make_uint4(o[0].x, o[0].y, o[1].x, o[1].y);
+}
+
+template <typename T>
+__device__ __forceinline__ typename Pair16<T>::V absmax16(typename Pair16<T>::V m, const uint4 (&v)[2]) {
+    using P = Pair16<T>;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        m = P::absmax(m, v[h].x);
+        m = P::absmax(m, v[h].y);
+        m = P::absmax(m, v[h].z);
+        m = P::absmax(m, v[h].w);
+    }
+    return m;
+}
+
+// The same with groups of 16 * TPG elements (TPG lanes): no reduction leaves the team.  One CTA per row
+// again: a grid-stride loop over groups loads, reduces and stores in turn and ran at 4.3 TB/s where
+// this runs at 6 (8192 x 4096).
+template <typename T, int MODE, int TPG>
+__global__ void __launch_bounds__(1024) group_row16_kernel(QuantArgs a) {
+    const int64_t row = blockIdx.x;
+    if (row >= resolve_rows(a)) return;
+    const int64_t src = source_row(a, row);
+    const int units = (int)(a.K / 16);
+    const uint4* x = reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(a.x) + (src >= 0 ? src : 0) * a.ld_x);
+    uint4* q = reinterpret_cast<uint4*>(a.q + row * a.ld_q);
+    uint4 v[ROW_UNITS][2];
+#pragma unroll
+    for (int j = 0; j < ROW_UNITS; ++j) {
+        const int u = threadIdx.x + j * blockDim.x;
+        const bool real = src >= 0 && u < units;
+        v[j][0] = real ? x[2 * u] : make_uint4(0u, 0u, 0u, 0u);
+        v[j][1] = real ? x[2 * u + 1] : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int j = 0; j < ROW_UNITS; ++j) {
+        const int u = threadIdx.x + j * blockDim.x;
+        float amax = Pair16<T>::reduce(absmax16<T>(typename Pair16<T>::V(), v[j]));
+#pragma unroll
+        for (int o = TPG / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        if (u >= units) continue;
+        const float s = make_scale<MODE>(amax, a.eps, a.pow2);
+        q[u] = quantize16<T, MODE, MODE>(v[j], make_divider<MODE>(s));
+        if (u % TPG == 0) a.s[row * a.s_row_stride + (u / TPG) * a.s_col_stride] = s;
+    }
+}
+
 template <typename T, int MODE>
 __global__ void __launch_bounds__(1024) row_quant16_kernel(QuantArgs a) {
     using P = Pair16<T>;
@@ -460,14 +517,7 @@ __global__ void __launch_bounds__(1024) row_quant16_kernel(QuantArgs a) {
     } else {
         typename P::V m2 = typename P::V();
 #pragma unroll
-        for (int j = 0; j < ROW_UNITS; ++j)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                m2 = P::absmax(m2, v[j][h].x);
-                m2 = P::absmax(m2, v[j][h].y);
-                m2 = P::absmax(m2, v[j][h].z);
-                m2 = P::absmax(m2, v[j][h].w);
-            }
+        for (int j = 0; j < ROW_UNITS; ++j) m2 = absmax16<T>(m2, v[j]);
         float amax = P::reduce(m2);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
@@ -487,21 +537,7 @@ __global__ void __launch_bounds__(1024) row_quant16_kernel(QuantArgs a) {
 #pragma unroll
     for (int j = 0; j < ROW_UNITS; ++j) {
         const int u = threadIdx.x + j * blockDim.x;
-        if (u >= units) break;
-        uint2 o[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t w[4] = {v[j][h].x, v[j][h].y, v[j][h].z, v[j][h].w};
-            float f[8];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                float lo, hi;
-                P::widen(w[i], lo, hi);
-                apply_divider2<DMODE>(lo, hi, d, f[2 * i], f[2 * i + 1]);
-            }
-            o[h] = pack_out8<MODE>(f);
-        }
-        q[u] = make_uint4(o[0].x, o[0].y, o[1].x, o[1].y);
+        if (u < units) q[u] = quantize16<T, MODE, DMODE>(v[j], d);
     }
 }
 
@@ -575,16 +611,23 @@ int launch_quant_t(const QuantArgs& a, cudaStream_t st) {
         return FG_OK;
     };
     if constexpr (sizeof(T) == 2) {
+        const int64_t threads = fg_cdiv(fg_cdiv(a.K, 16 * ROW_UNITS), 32) * 32;
+        auto by_row = [&](auto kernel) -> int {
+            kernel<<<(unsigned)a.rows, (unsigned)threads, 0, st>>>(a);
+            fg_count_launch(1);
+            FG_LAUNCH_CHECK();
+            return FG_OK;
+        };
         // 16-byte stores need 16-byte aligned output rows; otherwise the generic kernel below
         const bool q16 = ((uintptr_t)a.q % 16 == 0) && (a.ld_q % 16 == 0);
         if (q16 && a.meta_ids) {
-            if (a.group == 128) return small(group_quant16_kernel<T, MODE, 8, true>, 8);
-        } else if (q16) {
+            if (a.group == 128) return small(group_pack16_kernel<T, MODE>, 8);
+        } else if (q16 && threads <= 1024 && a.rows < (1ll << 31)) {
             switch (a.group) {
-                case 64: return small(group_quant16_kernel<T, MODE, 4, false>, 4);
-                case 128: return small(group_quant16_kernel<T, MODE, 8, false>, 8);
-                case 256: return small(group_quant16_kernel<T, MODE, 16, false>, 16);
-                case 512: return small(group_quant16_kernel<T, MODE, 32, false>, 32);
+                case 64: return by_row(group_row16_kernel<T, MODE, 4>);
+                case 128: return by_row(group_row16_kernel<T, MODE, 8>);
+                case 256: return by_row(group_row16_kernel<T, MODE, 16>);
+                case 512: return by_row(group_row16_kernel<T, MODE, 32>);
                 default: break;
             }
         }
