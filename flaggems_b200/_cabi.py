@@ -20,6 +20,8 @@ FG_OK = 0
 DTYPE_CODE = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
 DTYPE_E4M3 = 3  # output of fg_scaled_mm_fp8 only
 SCALE_SCALAR, SCALE_VECTOR, SCALE_BLOCK = 0, 1, 2
+(EXPERTS_BLOCK_FP8, EXPERTS_CHANNEL_FP8, EXPERTS_CHANNEL_INT8, EXPERTS_TENSOR_FP8, EXPERTS_16BIT,
+ EXPERTS_16BIT_SCALED) = range(6)
 
 _P = c_void_p
 _SIGS = {

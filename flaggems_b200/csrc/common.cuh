@@ -49,6 +49,53 @@ int fg_num_sms();
 // Index of the current device clamped to [0, 63]: the key of every per-device cache in the library.
 int fg_device_index();
 
+// Grouped expert GEMM with every option of the C-ABI forms, for the pipelines of this library.
+// gather_div > 0: a (row stride ld_a elements) and a_scale hold one row per token and route slot s
+// reads row s / gather_div through sorted_ids; 0: rows are in sorted order.
+struct FgGroupedGemm {
+    void* c;
+    const void *a, *w;
+    const float *a_scale, *w_scale;
+    const void* topk_w;
+    int topk_w_dtype;
+    int64_t topk_w_stride;
+    const int32_t *sorted_ids, *expert_ids, *num_post_pad;
+    int64_t a_rows;    // rows of a
+    int64_t max_rows;  // sorted rows
+    int64_t numel;
+    int gather_div;
+    int a_contiguous;  // with gather_div = 1: the slots of a block are consecutive rows of a
+    int num_experts;
+    int64_t N, K, ld_a, ld_as, ld_c;  // ld_as: block scales only
+    int operand;  // 0 e4m3, 1 int8, 2 bf16, 3 fp16
+    int block_rows, scale_mode, a_scale_per_row, fuse_silu, scatter, mul_weight, out_dtype;
+    const float* bias;  // fp32, added before the cast; bias_stride elements between the rows of consecutive experts
+    int64_t bias_stride;
+    const int32_t* dest;
+    int64_t dest_stride;
+    void* const* peer_out;
+    int n_peers;
+    int64_t peer_rows;
+};
+int fg_grouped_gemm(const FgGroupedGemm& g, cudaStream_t stream);
+
+// sorted_ids / expert_ids / num_post_pad of rows grouped by the ends `offs`, padded to `block` per group.
+int fg_group_tiles(const int32_t* offs, int num_groups, int64_t rows, int block, int32_t* sorted_ids, int64_t max_pad,
+                   int32_t* expert_ids, int64_t n_blocks, int32_t* num_post_pad, cudaStream_t stream);
+
+// x[0:n] = 1
+int fg_fill_ones(float* x, int64_t n, cudaStream_t stream);
+
+// Contiguous rows [*, K] -> quantised rows [rows, K] and scales, optionally through row_index (output row
+// r takes row row_index[r] / index_div; index_div = 0: row r itself) and with the row count on the
+// device.  Output rows whose index is outside [0, index_limit) are padding and become zeros.
+// FG_QUANT_TENSOR: tensor_scale is the given scale, or with scale_out != NULL the
+// amax it is derived from.
+enum { FG_QUANT_GROUP128 = 0, FG_QUANT_TOKEN = 1, FG_QUANT_INT8 = 2, FG_QUANT_TENSOR = 3 };
+int fg_quant_rows(int kind, const void* x, int x_dtype, void* q, float* s, const float* tensor_scale, float* scale_out, int64_t rows,
+                  int64_t K, const int32_t* row_index, int32_t index_div, int32_t index_limit, const int32_t* n_rows_dev,
+                  cudaStream_t st);
+
 // Adds n to the process-wide count of kernels launched by this library.
 void fg_count_launch(int n);
 

@@ -85,6 +85,10 @@ struct GemmParams {
     int block_rows;  // grouped: rows per m-tile (TMA box rows of A), <= 128
     int a_box_rows;  // dense: TMA box rows of A (128, or fewer when M is small)
     int64_t numel;
+    // Grouped, gather_div > 0: A (and its per-row scales) holds one row per token and route slot s reads
+    // row s / gather_div through sorted_ids; gather_div == 0: rows of A are already in sorted order.
+    int gather_div;
+    int a_contiguous;  // gather_div = 1 and the slots of a block are consecutive rows of A: one box from the first
     int scatter, mul_weight;
     const void* topk_w;
     int topk_w_dtype;
@@ -400,7 +404,11 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
       if constexpr (C::REBALANCE_REGS) setmaxnreg_dec<C::REGS_PRODUCER>();
       if (warp == 0) {
         // ------------------------------- TMA producer -------------------------------------
-        if (lane == 0) {
+        // Gathered A rows (few per tile, see the callers) are fetched by the whole warp: lane l names rows 4l .. 4l + 3 of the tile to one
+        // tile::gather4, and lanes whose four rows are all padding fetch nothing (their rows of the
+        // stage keep old bytes, which only reach accumulator rows nobody reads).
+        const bool gather = p.gather_div > 0 && !p.a_contiguous;
+        if (lane == 0 || gather) {
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -409,11 +417,26 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                 const TileCoord tc = tile_coord(t, num_m, num_n);
                 const int expert = p.grouped ? p.expert_ids[tc.m_blk] : 0;
                 if (expert < 0) continue;
-                const int m0 = tc.m_blk * a_rows_step + (int)cta_rank * BLOCK_M;
+                int m0 = tc.m_blk * a_rows_step + (int)cta_rank * BLOCK_M;
                 const int n0 = tc.n_blk * OUT_TILE_N;
+                if (p.a_contiguous) m0 = p.sorted_ids[m0];
+                int4 rows = make_int4(0, 0, 0, 0);
+                bool mine = false;
+                uint32_t tx = stage_tx;
+                if (gather) {
+                    const int4 sid = *reinterpret_cast<const int4*>(p.sorted_ids + m0 + 4 * lane);
+                    auto token = [&](int s) {
+                        const bool real = s >= 0 && s < p.numel;
+                        mine |= real;
+                        return real ? s / p.gather_div : 0;
+                    };
+                    rows = make_int4(token(sid.x), token(sid.y), token(sid.z), token(sid.w));
+                    tx = (uint32_t)(__popc(__ballot_sync(0xffffffffu, mine)) * 4 * BLOCK_K + C::B_BYTES);
+                }
                 for (int kb = kb_begin; kb < kb_end; ++kb) {
                     FG_PROF_T0(tw);
                     ok = mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, 1);
+                    if (gather) ok = __all_sync(0xffffffffu, ok);
                     FG_PROF_ADD(prof_wait, tw);
                     if (!ok) break;
                     uint8_t* sa = smem + stage * C::STAGE_BYTES;
@@ -432,14 +455,20 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                         }
                         continue;
                     }
-                    mbar_arrive_expect_tx(&full_bar[stage], stage_tx);
-                    tma_load_2d(sa, &tm_a, &full_bar[stage], kb * BLOCK_K, m0);
-                    if constexpr (FUSE_SILU) {
-                        tma_load_3d(sb, &tm_b, &full_bar[stage], kb * BLOCK_K, n0, expert);
-                        tma_load_3d(sb + (BN / 2) * BLOCK_K, &tm_b, &full_bar[stage], kb * BLOCK_K, p.N / 2 + n0,
-                                    expert);
-                    } else {
-                        tma_load_3d(sb, &tm_b, &full_bar[stage], kb * BLOCK_K, n0, expert);
+                    if (lane == 0) {
+                        mbar_arrive_expect_tx(&full_bar[stage], tx);
+                        if (!gather) tma_load_2d(sa, &tm_a, &full_bar[stage], kb * BLOCK_K, m0);
+                        if constexpr (FUSE_SILU) {
+                            tma_load_3d(sb, &tm_b, &full_bar[stage], kb * BLOCK_K, n0, expert);
+                            tma_load_3d(sb + (BN / 2) * BLOCK_K, &tm_b, &full_bar[stage], kb * BLOCK_K, p.N / 2 + n0,
+                                        expert);
+                        } else {
+                            tma_load_3d(sb, &tm_b, &full_bar[stage], kb * BLOCK_K, n0, expert);
+                        }
+                    }
+                    if (gather) {
+                        __syncwarp();
+                        if (mine) tma_gather4(sa + lane * 4 * BLOCK_K, &tm_a, &full_bar[stage], kb * BLOCK_K, rows);
                     }
                     if (++stage == STAGES) {
                         stage = 0;
@@ -681,13 +710,17 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
 
             // Where this thread's row goes, and whether it is written at all.
             bool row_ok;
-            int64_t out_row = row;
+            int64_t out_row = row, src_row = row;
             float weight = 1.0f;
             if (p.grouped) {
                 row_ok = r_in_tile < p.block_rows;
-                if (row_ok && (p.scatter || p.mul_weight)) {
+                if (row_ok && (p.scatter || p.mul_weight || p.gather_div > 0)) {
                     const int32_t sid = p.sorted_ids[row];
                     const bool real = sid >= 0 && sid < p.numel;
+                    if (p.gather_div > 0) {
+                        row_ok = real;
+                        src_row = real ? sid / p.gather_div : 0;
+                    }
                     if (p.scatter) {
                         row_ok = real;
                         out_row = sid;
@@ -728,7 +761,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                 }
                 continue;
             }
-            const int64_t srow = p.grouped ? row : (row < p.M ? row : p.M - 1);  // row used for scale loads
+            const int64_t srow = p.grouped ? src_row : (row < p.M ? row : p.M - 1);  // row used for scale loads
 
             if constexpr (!BLOCK_SCALED) {
                 const uint32_t buf = acc_iter & 1u;
@@ -1295,7 +1328,7 @@ int launch_gemm(GemmParams& p, const void* a, int64_t a_rows, int64_t ld_a, cons
     const int esz = out_elem_size(p.out_dtype);
     p.c_vec_ok = ((uintptr_t)p.c % 16 == 0) && ((p.ld_c * esz) % 16 == 0);
 
-    const int64_t m_tiles = p.grouped ? a_rows / p.block_rows : fg_cdiv(p.M, BLOCK_M);
+    const int64_t m_tiles = p.grouped ? p.M / p.block_rows : fg_cdiv(p.M, BLOCK_M);
     const int sms = fg_num_sms();
     // Tile width.  One K block costs a CTA about the same time whatever the width (an MMA with
     // M = 128 streams 128 rows of A however few columns it has), so the widest tile wins as long
@@ -1350,7 +1383,7 @@ int launch_gemm(GemmParams& p, const void* a, int64_t a_rows, int64_t ld_a, cons
 
     CUtensorMap ta, tb;
     int rc = make_map(&ta, a, (uint64_t)p.K, (uint64_t)a_rows, 1, (uint64_t)ld_a, 0,
-                      (uint32_t)(p.grouped ? p.block_rows : p.a_box_rows), 2);
+                      (uint32_t)(p.gather_div > 0 && !p.a_contiguous ? 1 : p.grouped ? p.block_rows : p.a_box_rows), 2);
     if (rc != FG_OK) return rc;
     rc = make_map(&tb, b, (uint64_t)p.K, (uint64_t)p.N, (uint64_t)num_experts, (uint64_t)ld_b,
                   (uint64_t)ld_b * (uint64_t)p.N, (uint32_t)((fuse_silu || pair) ? bn / 2 : bn), 3);
@@ -1509,70 +1542,90 @@ int fg_grouped_gemm_fp8_bias(void* c, const void* a, const void* w, const float*
                "null pointer");
     FG_REQUIRE(dtype_ok(out_dtype), FG_ERR_INVALID_ARGUMENT, "bad out_dtype %d", out_dtype);
     FG_REQUIRE(N < (1ll << 31) && K < (1ll << 31), FG_ERR_UNSUPPORTED, "dimension too large");
-    if (max_rows == 0) return FG_OK;
-    GemmParams p{};
-    p.M = max_rows / BLOCK_M * BLOCK_M; p.N = (int)N; p.K = (int)K; p.n_out = (int)N;
-    p.c = c; p.ld_c = ld_c; p.out_dtype = out_dtype;
-    p.sa = a_scale; p.sb = w_scale; p.sa_mode = FG_SCALE_VECTOR; p.sb_mode = FG_SCALE_VECTOR; p.sb_stride_e = N;
-    p.bias = bias; p.bias_dtype = FG_DTYPE_F32; p.bias_stride_e = bias_stride_g; p.bias_after_round = 0;
-    p.grouped = 1; p.sorted_ids = sorted_ids; p.expert_ids = expert_ids; p.num_post_pad = num_post_pad;
-    p.block_rows = BLOCK_M; p.numel = numel; p.scatter = 1; p.mul_weight = 0; p.topk_w_stride = 1;
-    return launch_gemm(p, a, p.M, ld_a, w, num_groups, K, false, false, (cudaStream_t)stream);
+    FgGroupedGemm g{};
+    g.c = c; g.a = a; g.w = w; g.a_scale = a_scale; g.w_scale = w_scale; g.bias = bias; g.bias_stride = bias_stride_g;
+    g.sorted_ids = sorted_ids; g.expert_ids = expert_ids; g.num_post_pad = num_post_pad;
+    g.max_rows = max_rows; g.numel = numel; g.num_experts = num_groups; g.N = N; g.K = K; g.ld_a = ld_a; g.ld_c = ld_c;
+    g.block_rows = BLOCK_M; g.scale_mode = FG_SCALE_VECTOR; g.scatter = 1; g.out_dtype = out_dtype;
+    return fg_grouped_gemm(g, (cudaStream_t)stream);
 }
 
-static int grouped_gemm_common(int int8, void* c, const void* a, const void* w, const float* a_scale, const float* w_scale,
-                            const void* topk_weights, int topk_w_dtype, int64_t topk_w_stride,
-                            const int32_t* sorted_ids,
-                            const int32_t* expert_ids, const int32_t* num_post_pad, int64_t max_rows, int64_t numel,
-                            int num_experts, int64_t N, int64_t K, int64_t ld_a, int64_t ld_c, int block_rows,
-                            int scale_mode, int a_scale_per_row, int fuse_silu, int scatter, int mul_weight,
-                            int out_dtype, const int32_t* dest, int64_t dest_stride, void* const* peer_out, int n_peers,
-                            int64_t peer_rows, void* stream) {
-    FG_REQUIRE(max_rows >= 0 && N > 0 && K > 0 && num_experts > 0, FG_ERR_INVALID_ARGUMENT, "bad sizes");
-    FG_REQUIRE((c || n_peers > 0) && a && w && a_scale && w_scale && sorted_ids && expert_ids && num_post_pad,
+}  // extern "C"
+
+int fg_grouped_gemm(const FgGroupedGemm& g, cudaStream_t stream) {
+    FG_REQUIRE(g.max_rows >= 0 && g.N > 0 && g.K > 0 && g.num_experts > 0, FG_ERR_INVALID_ARGUMENT, "bad sizes");
+    FG_REQUIRE((g.c || g.n_peers > 0) && g.a && g.w && g.a_scale && g.w_scale && g.sorted_ids && g.expert_ids && g.num_post_pad,
                FG_ERR_INVALID_ARGUMENT, "null pointer");
-    FG_REQUIRE(n_peers >= 0 && n_peers <= 8 &&
-                   (n_peers == 0 || (dest && peer_out && scatter && dest_stride >= 2 && peer_rows > 0)),
+    FG_REQUIRE(g.n_peers >= 0 && g.n_peers <= 8 &&
+                   (g.n_peers == 0 || (g.dest && g.peer_out && g.scatter && g.dest_stride >= 2 && g.peer_rows > 0)),
                FG_ERR_INVALID_ARGUMENT,
                "peer scatter needs 1..8 peers, scatter mode, a (slot, rank) table and the peers' row capacity");
-    FG_REQUIRE(dtype_ok(out_dtype), FG_ERR_INVALID_ARGUMENT, "bad out_dtype %d", out_dtype);
-    FG_REQUIRE(block_rows >= 8 && block_rows <= 128 && block_rows % 8 == 0, FG_ERR_UNSUPPORTED,
-               "block_rows %d must be a multiple of 8 in [8, 128]", block_rows);
-    FG_REQUIRE(!mul_weight || (topk_weights && dtype_ok(topk_w_dtype)), FG_ERR_INVALID_ARGUMENT,
+    FG_REQUIRE(dtype_ok(g.out_dtype), FG_ERR_INVALID_ARGUMENT, "bad out_dtype %d", g.out_dtype);
+    FG_REQUIRE(g.block_rows >= 8 && g.block_rows <= 128 && g.block_rows % 8 == 0, FG_ERR_UNSUPPORTED,
+               "block_rows %d must be a multiple of 8 in [8, 128]", g.block_rows);
+    FG_REQUIRE(!g.mul_weight || (g.topk_w && dtype_ok(g.topk_w_dtype)), FG_ERR_INVALID_ARGUMENT,
                "mul_weight needs topk_weights");
-    FG_REQUIRE(N < (1ll << 31) && K < (1ll << 31), FG_ERR_UNSUPPORTED, "dimension too large");
-    FG_REQUIRE(!fuse_silu || N % 2 == 0, FG_ERR_INVALID_ARGUMENT, "fused SiLU needs an even N");
-    const bool block = scale_mode == FG_SCALE_BLOCK;
-    FG_REQUIRE(!(block && fuse_silu) || (N / 2) % 128 == 0, FG_ERR_UNSUPPORTED,
+    FG_REQUIRE(g.N < (1ll << 31) && g.K < (1ll << 31), FG_ERR_UNSUPPORTED, "dimension too large");
+    FG_REQUIRE(!g.fuse_silu || g.N % 2 == 0, FG_ERR_INVALID_ARGUMENT, "fused SiLU needs an even N");
+    const bool block = g.scale_mode == FG_SCALE_BLOCK;
+    FG_REQUIRE(!(block && g.fuse_silu) || (g.N / 2) % 128 == 0, FG_ERR_UNSUPPORTED,
                "fused SiLU with block scales needs the intermediate size %lld to be a multiple of 128",
-               (long long)(N / 2));
-    if (max_rows == 0) return FG_OK;
-    if (int8 >= 2) {  // 16-bit operands: the kernel counts K and the operand row strides in bytes
+               (long long)(g.N / 2));
+    FG_REQUIRE(g.gather_div == 0 || (g.gather_div > 0 && g.block_rows == BLOCK_M && (uintptr_t)g.sorted_ids % 16 == 0),
+               FG_ERR_INVALID_ARGUMENT, "gathered rows need 128-row blocks and 16-byte aligned sorted_ids");
+    if (g.max_rows == 0) return FG_OK;
+    int64_t K = g.K, ld_a = g.ld_a;
+    if (g.operand >= 2) {  // 16-bit operands: the kernel counts K and the operand row strides in bytes
         FG_REQUIRE(!block && K % 8 == 0 && 2 * K < (1ll << 31), FG_ERR_UNSUPPORTED,
                    "16-bit operands take per-tensor or per-row x per-column scales and K a multiple of 8");
         K *= 2;
         ld_a *= 2;
     }
     GemmParams p{};
-    p.M = max_rows / block_rows * block_rows; p.N = (int)N; p.K = (int)K; p.n_out = fuse_silu ? (int)(N / 2) : (int)N;
-    p.c = c; p.ld_c = ld_c; p.out_dtype = out_dtype;
-    p.sa = a_scale; p.sb = w_scale;
+    p.M = g.max_rows / g.block_rows * g.block_rows; p.N = (int)g.N; p.K = (int)K; p.n_out = (int)(g.fuse_silu ? g.N / 2 : g.N);
+    p.c = g.c; p.ld_c = g.ld_c; p.out_dtype = g.out_dtype;
+    p.sa = g.a_scale; p.sb = g.w_scale;
     if (block) {
-        const int64_t kb = fg_cdiv(K, 128), nb = fg_cdiv(N, 128);
-        p.ld_as = kb; p.as_stride_k = 1; p.bs_stride_k = 1; p.bs_stride_n = kb; p.bs_stride_e = kb * nb;
+        const int64_t kb = fg_cdiv(K, 128), nb = fg_cdiv(g.N, 128);
+        p.ld_as = g.ld_as; p.as_stride_k = 1; p.bs_stride_k = 1; p.bs_stride_n = kb; p.bs_stride_e = kb * nb;
     } else {
-        p.sa_mode = (scale_mode == FG_SCALE_VECTOR || a_scale_per_row) ? FG_SCALE_VECTOR : FG_SCALE_SCALAR;
-        p.sb_mode = scale_mode == FG_SCALE_VECTOR ? FG_SCALE_VECTOR : FG_SCALE_SCALAR;
-        p.sb_stride_e = N;
+        p.sa_mode = (g.scale_mode == FG_SCALE_VECTOR || g.a_scale_per_row) ? FG_SCALE_VECTOR : FG_SCALE_SCALAR;
+        p.sb_mode = g.scale_mode == FG_SCALE_VECTOR ? FG_SCALE_VECTOR : FG_SCALE_SCALAR;
+        p.sb_stride_e = g.N;
     }
-    p.grouped = 1; p.int8 = int8; p.sorted_ids = sorted_ids; p.expert_ids = expert_ids; p.num_post_pad = num_post_pad;
-    p.block_rows = block_rows; p.numel = numel; p.scatter = scatter; p.mul_weight = mul_weight;
-    p.topk_w = topk_weights; p.topk_w_dtype = topk_w_dtype; p.topk_w_stride = topk_w_stride > 0 ? topk_w_stride : 1;
-    p.dest = dest; p.dest_stride = dest_stride; p.n_peers = n_peers; p.peer_rows = peer_rows;
-    for (int i = 0; i < n_peers; ++i) p.peer_out[i] = peer_out[i];
-    if (n_peers > 0 && !c) p.c = peer_out[0];
-    return launch_gemm(p, a, p.M, ld_a, w, num_experts, K, block, fuse_silu != 0, (cudaStream_t)stream);
+    p.grouped = 1; p.int8 = g.operand;
+    p.sorted_ids = g.sorted_ids; p.expert_ids = g.expert_ids; p.num_post_pad = g.num_post_pad;
+    p.block_rows = g.block_rows; p.numel = g.numel; p.gather_div = g.gather_div; p.a_contiguous = g.a_contiguous;
+    p.scatter = g.scatter; p.mul_weight = g.mul_weight;
+    p.topk_w = g.topk_w; p.topk_w_dtype = g.topk_w_dtype; p.topk_w_stride = g.topk_w_stride > 0 ? g.topk_w_stride : 1;
+    p.bias = g.bias; p.bias_dtype = FG_DTYPE_F32; p.bias_stride_e = g.bias_stride;
+    p.dest = g.dest; p.dest_stride = g.dest_stride; p.n_peers = g.n_peers; p.peer_rows = g.peer_rows;
+    for (int i = 0; i < g.n_peers; ++i) p.peer_out[i] = g.peer_out[i];
+    if (g.n_peers > 0 && !g.c) p.c = g.peer_out[0];
+    return launch_gemm(p, g.a, g.gather_div > 0 ? g.a_rows : p.M, ld_a, g.w, g.num_experts, K, block, g.fuse_silu != 0, stream);
 }
+
+// The C-ABI forms: rows of a in sorted order.
+static int grouped_gemm_common(int operand, void* c, const void* a, const void* w, const float* a_scale, const float* w_scale,
+                               const void* topk_weights, int topk_w_dtype, int64_t topk_w_stride,
+                               const int32_t* sorted_ids, const int32_t* expert_ids, const int32_t* num_post_pad,
+                               int64_t max_rows, int64_t numel, int num_experts, int64_t N, int64_t K, int64_t ld_a,
+                               int64_t ld_c, int block_rows, int scale_mode, int a_scale_per_row, int fuse_silu,
+                               int scatter, int mul_weight, int out_dtype, const int32_t* dest, int64_t dest_stride,
+                               void* const* peer_out, int n_peers, int64_t peer_rows, void* stream) {
+    FgGroupedGemm g{};
+    g.c = c; g.a = a; g.w = w; g.a_scale = a_scale; g.w_scale = w_scale;
+    g.topk_w = topk_weights; g.topk_w_dtype = topk_w_dtype; g.topk_w_stride = topk_w_stride;
+    g.sorted_ids = sorted_ids; g.expert_ids = expert_ids; g.num_post_pad = num_post_pad;
+    g.max_rows = max_rows; g.numel = numel; g.num_experts = num_experts;
+    g.N = N; g.K = K; g.ld_a = ld_a; g.ld_as = fg_cdiv(K, 128); g.ld_c = ld_c; g.operand = operand;
+    g.block_rows = block_rows; g.scale_mode = scale_mode; g.a_scale_per_row = a_scale_per_row; g.fuse_silu = fuse_silu;
+    g.scatter = scatter; g.mul_weight = mul_weight; g.out_dtype = out_dtype;
+    g.dest = dest; g.dest_stride = dest_stride; g.peer_out = peer_out; g.n_peers = n_peers; g.peer_rows = peer_rows;
+    return fg_grouped_gemm(g, (cudaStream_t)stream);
+}
+
+extern "C" {
 
 int fg_moe_grouped_gemm_fp8_peer(void* c, const void* a, const void* w, const float* a_scale, const float* w_scale,
                                  const void* topk_weights, int topk_w_dtype, int64_t topk_w_stride,

@@ -469,12 +469,54 @@ PyObject* moe_sum(PyObject*, PyObject* const* p, Py_ssize_t n) {
     });
 }
 
+// fused_experts(hidden, w1, w2, topk_weights, topk_ids, out, mode, w1_scale, w2_scale, a1_scale, a2_scale,
+//               num_experts, expert_map, tokens per chunk) -> out.  The caller has checked shapes, types and
+// layouts; scales, map and the two activation scales may be None.
+PyObject* fused_experts(PyObject*, PyObject* const* p, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        int64_t mode, experts, chunk;
+        if (n != 14 || !py_int(p[6], &mode) || !py_int(p[11], &experts) || !py_int(p[13], &chunk)) return none();
+        const at::Tensor *x = cuda_tensor(p[0]), *w1 = cuda_tensor(p[1]), *w2 = cuda_tensor(p[2]), *tw = cuda_tensor(p[3]),
+                         *ids = cuda_tensor(p[4]), *out = cuda_tensor(p[5]);
+        if (!x || !w1 || !w2 || !tw || !ids || !out) return none();
+        const float* f[4] = {nullptr, nullptr, nullptr, nullptr};
+        for (int i = 0; i < 4; ++i) {
+            if (p[7 + i] == Py_None) continue;
+            const at::Tensor* s = cuda_tensor(p[7 + i]);
+            if (!s || s->scalar_type() != ScalarType::Float) return none();
+            f[i] = static_cast<const float*>(s->data_ptr());
+        }
+        const at::Tensor* map = nullptr;
+        if (p[12] != Py_None && !(map = cuda_tensor(p[12]))) return none();
+        const int64_t t = x->size(0), h = x->size(1), inter = w2->size(2), topk = ids->size(1);
+        const int code = dtype_code(x->scalar_type()), esz = (int)x->element_size();
+        const bool i64 = ids->scalar_type() == ScalarType::Long;
+        c10::cuda::CUDAGuard guard(x->device());
+        const int64_t most = t < chunk ? t : chunk;
+        const int64_t need = fg_fused_experts_workspace_bytes((int)mode, most, (int)topk, (int)experts, h, inter, code);
+        at::Tensor ws = empty({need}, ScalarType::Byte, *x);
+        for (int64_t b = 0; b < t; b += chunk) {
+            const int64_t rows = t - b < chunk ? t - b : chunk;
+            const int rc = fg_fused_experts(
+                static_cast<char*>(out->data_ptr()) + b * h * esz, static_cast<const char*>(x->data_ptr()) + b * h * esz, code,
+                static_cast<const char*>(ids->data_ptr()) + b * topk * (i64 ? 8 : 4), i64,
+                static_cast<const char*>(tw->data_ptr()) + b * topk * tw->element_size(), dtype_code(tw->scalar_type()), rows,
+                (int)topk, w1->data_ptr(), w2->data_ptr(), f[0], f[1], f[2], f[3], (int)mode, (int)experts, (int)w1->size(0),
+                map ? static_cast<const int32_t*>(map->data_ptr()) : nullptr, map ? (int)map->numel() : 0, h, inter, nullptr,
+                ws.data_ptr(), need, stream_of(*x));
+            if (rc != FG_OK) return raise_rc(rc);
+        }
+        Py_INCREF(p[5]);
+        return p[5];
+    });
+}
+
 #define FG_METHOD(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
     FG_METHOD(group_quant), FG_METHOD(act_quant),    FG_METHOD(token_quant), FG_METHOD(tensor_quant),
     FG_METHOD(block_mm),    FG_METHOD(scaled_mm),    FG_METHOD(scaled_mm_new), FG_METHOD(grouped_mm),
     FG_METHOD(topk_softmax), FG_METHOD(grouped_topk), FG_METHOD(moe_align),  FG_METHOD(silu_mul),
-    FG_METHOD(moe_sum),     {nullptr, nullptr, 0, nullptr}};
+    FG_METHOD(moe_sum),     FG_METHOD(fused_experts), {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fg_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

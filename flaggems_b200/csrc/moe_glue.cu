@@ -358,6 +358,61 @@ __global__ void __launch_bounds__(256) group_ids_kernel(const int32_t* __restric
     }
 }
 
+// The alignment tables of rows that are already grouped (group g = rows [offs[g-1], offs[g])): the same
+// sorted_ids / expert_ids / num_post_pad as moe_align on the rows' group ids, straight from the ends.
+// Every CTA scans the padded group sizes for itself and fills its share of sorted_ids.
+__global__ void __launch_bounds__(ALIGN_THREADS, 1) group_tiles_kernel(const int32_t* __restrict__ offs, int num_groups,
+                                                                       int32_t rows, int32_t block, int32_t* __restrict__ sorted_ids,
+                                                                       int64_t max_pad, int32_t* __restrict__ expert_ids,
+                                                                       int64_t n_blocks, int32_t* __restrict__ num_post_pad) {
+    __shared__ int32_t first[ALIGN_THREADS], pad_first[ALIGN_THREADS + 1], scan_tmp[ALIGN_WARPS];
+    const int g = threadIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int32_t lo = 0, count = 0;
+    if (g < num_groups) {
+        lo = g > 0 ? min(max(offs[g - 1], 0), rows) : 0;
+        count = max(min(offs[g], rows) - lo, 0);
+    }
+    const int32_t padded = (count + block - 1) / block * block;
+    int32_t incl = padded;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) scan_tmp[warp] = incl;
+    __syncthreads();
+    int32_t before = 0;
+    for (int w = 0; w < warp; ++w) before += scan_tmp[w];
+    first[g] = lo;
+    pad_first[g] = before + incl - padded;
+    if (g == ALIGN_THREADS - 1) pad_first[ALIGN_THREADS] = before + incl;
+    __syncthreads();
+    const int32_t total = pad_first[ALIGN_THREADS];
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < max_pad; p += (int64_t)gridDim.x * blockDim.x) {
+        int32_t id = rows;
+        if (p < total) {
+            int a = 0, b = num_groups;  // last group whose padded range starts at or before p
+            while (b - a > 1) {
+                const int mid = (a + b) >> 1;
+                if (pad_first[mid] <= p) a = mid;
+                else b = mid;
+            }
+            const int32_t r = first[a] + (int32_t)(p - pad_first[a]);
+            const int32_t end = min(offs[a], rows);
+            if (r < end) id = r;
+            if (p % block == 0) expert_ids[p / block] = a;
+        } else if (p % block == 0 && p / block < n_blocks) {
+            expert_ids[p / block] = -1;
+        }
+        sorted_ids[p] = id;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) num_post_pad[0] = total;
+}
+
+__global__ void __launch_bounds__(256) fill_ones_kernel(float* __restrict__ x, int64_t n) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) x[i] = 1.0f;
+}
+
 unsigned grid_for(int64_t work_items, int per_block) {
     int64_t b = fg_cdiv(work_items, per_block);
     const int64_t cap = (int64_t)fg_num_sms() * 16;
@@ -462,6 +517,29 @@ int fg_group_ids_from_offsets(const int32_t* offs, int num_groups, int64_t rows,
     FG_LAUNCH_CHECK();
     return FG_OK;
 }
+
+}  // extern "C"
+
+int fg_fill_ones(float* x, int64_t n, cudaStream_t stream) {
+    fill_ones_kernel<<<grid_for(n, 256), 256, 0, stream>>>(x, n);
+    fg_count_launch(1);
+    FG_LAUNCH_CHECK();
+    return FG_OK;
+}
+
+int fg_group_tiles(const int32_t* offs, int num_groups, int64_t rows, int block, int32_t* sorted_ids, int64_t max_pad,
+                   int32_t* expert_ids, int64_t n_blocks, int32_t* num_post_pad, cudaStream_t stream) {
+    FG_REQUIRE(num_groups > 0 && num_groups <= ALIGN_THREADS && block > 0, FG_ERR_UNSUPPORTED, "at most %d groups", ALIGN_THREADS);
+    FG_REQUIRE(rows + (int64_t)num_groups * block < (1ll << 31), FG_ERR_UNSUPPORTED, "too many rows");
+    const int64_t blocks = fg_cdiv(max_pad, ALIGN_THREADS);
+    group_tiles_kernel<<<(unsigned)(blocks < fg_num_sms() ? blocks : fg_num_sms()), ALIGN_THREADS, 0, stream>>>(
+        offs, num_groups, (int32_t)rows, block, sorted_ids, max_pad, expert_ids, n_blocks, num_post_pad);
+    fg_count_launch(1);
+    FG_LAUNCH_CHECK();
+    return FG_OK;
+}
+
+extern "C" {
 
 int fg_silu_and_mul(const void* x, const void* y, void* out, int64_t M, int64_t N, int64_t ld_x, int64_t ld_y,
                     int64_t ld_out, int dtype, void* stream) {

@@ -1,8 +1,16 @@
-// Routed-expert pipeline of the block-FP8 MoE layer as ONE host call: align -> gather (and
-// quantise) into expert-sorted padded order -> grouped GEMM1 with fused SiLU*up -> group
-// quantisation -> grouped GEMM2 with the router weight.  Five launches issued back to back from
-// C++, so the host cost of a layer step does not grow with the number of kernels.  All scratch
-// lives in a caller-provided workspace; nothing is allocated here.
+// MoE pipelines as ONE host call each: align -> quantise -> grouped GEMM1 with fused SiLU*up -> quantise ->
+// grouped GEMM2 with the router weight (-> top-k sum), issued back to back from C++ into a caller's
+// workspace.
+//
+// Two orders of the rows between the launches:
+//   gathered  (few rows per expert: decode) the GEMMs fetch their A rows through sorted_ids with
+//             tile::gather4 and store in route-slot order: nothing touches padding rows.  The copy into
+//             expert order and the padding cost 60 us of a 32-token DeepSeek-V3 step.
+//   sorted    (otherwise) rows are laid out in expert order, padded to 128 per expert, and fetched as
+//             TMA boxes.  Padding rows are zeros all the way: written once, they cost less than the tensor
+//             power that stale bytes in their place draw (2 % of a step under the power cap).  A gather4 of four 128-byte rows takes ~70 cycles whatever the rows, so a full tile
+//             of them (32 per K block) is four times slower than its MMAs: the line lies at 32 rows per
+//             expert, where eight lanes' gathers still hide behind the weight stream.
 #include <mutex>
 
 #include "common.cuh"
@@ -18,39 +26,53 @@ constexpr int TILE_ROWS = 128;
 
 inline int64_t align_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
 
+// What an expert pipeline keeps between its launches.
 struct Workspace {
     int32_t* sorted_ids;
     int32_t* expert_ids;
     int32_t* post_pad;
-    uint8_t* a1;
+    float* scalars;  // per-tensor modes: amax and scale of both GEMMs' inputs; 16-bit mode: unit scales
+    uint8_t* a1;     // input rows of GEMM1: quantised, or 16-bit copies in expert order
     float* a1s;
-    uint8_t* act;
-    uint8_t* a2;
+    uint8_t* act;    // GEMM1's output
+    uint8_t* a2;     // the same quantised
     float* a2s;
+    uint8_t* routed; // GEMM2's output, one row per route slot
     int64_t max_pad, n_blocks, rows, bytes;
 };
 
-Workspace carve(void* base, int64_t n_in, int num_experts, int64_t H, int64_t I, int out_esz) {
-    Workspace w{};
-    w.max_pad = n_in + (int64_t)num_experts * (TILE_ROWS - 1);
-    w.n_blocks = fg_cdiv(w.max_pad, TILE_ROWS);
-    w.rows = w.max_pad / TILE_ROWS * TILE_ROWS;
-    uint8_t* p = reinterpret_cast<uint8_t*>(base);
-    int64_t off = 0;
-    auto take = [&](int64_t bytes) {
+struct Carver {
+    uint8_t* p;
+    int64_t off;
+    uint8_t* take(int64_t bytes) {
         uint8_t* r = p ? p + off : nullptr;
         off += align_up(bytes, 256);
         return r;
-    };
-    w.sorted_ids = (int32_t*)take(4 * w.max_pad);
-    w.expert_ids = (int32_t*)take(4 * w.n_blocks);
-    w.post_pad = (int32_t*)take(256);
-    w.a1 = take(w.rows * H);
-    w.a1s = (float*)take(4 * w.rows * (H / 128));
-    w.act = take(w.rows * I * out_esz);
-    w.a2 = take(w.rows * I);
-    w.a2s = (float*)take(4 * w.rows * (I / 128));
-    w.bytes = off;
+    }
+};
+
+// Sorted rows of `slots` route slots: every expert padded to the tile, and no more than one tile per slot.
+void carve_tables(Carver& c, Workspace& w, int64_t slots, int num_experts) {
+    w.max_pad = slots + (int64_t)num_experts * (TILE_ROWS - 1);
+    if (slots * TILE_ROWS < w.max_pad) w.max_pad = slots * TILE_ROWS;
+    w.n_blocks = fg_cdiv(w.max_pad, TILE_ROWS);
+    w.rows = w.max_pad / TILE_ROWS * TILE_ROWS;
+    w.sorted_ids = (int32_t*)c.take(4 * w.max_pad);
+    w.expert_ids = (int32_t*)c.take(4 * w.n_blocks);
+    w.post_pad = (int32_t*)c.take(256);
+}
+
+// Routed block-FP8 pipeline.
+Workspace carve(void* base, int64_t slots, int num_experts, int64_t H, int64_t I, int esz) {
+    Workspace w{};
+    Carver c{reinterpret_cast<uint8_t*>(base), 0};
+    carve_tables(c, w, slots, num_experts);
+    w.a1 = c.take(w.rows * H);
+    w.a1s = (float*)c.take(4 * w.rows * (H / 128));
+    w.act = c.take(w.rows * I * esz);
+    w.a2 = c.take(w.rows * I);
+    w.a2s = (float*)c.take(4 * w.rows * (I / 128));
+    w.bytes = c.off;
     return w;
 }
 
@@ -63,22 +85,108 @@ int check_dims(int64_t n_in, int num_experts, int64_t H, int64_t I, int out_dtyp
     return FG_OK;
 }
 
-// GEMM1 -> quant -> GEMM2 on rows already in sorted order in ws.a1 / ws.a1s.
-int run_gemms(void* y, const Workspace& ws, int64_t n_in, const void* w1, const void* w2, const float* s1,
-              const float* s2, int num_experts, int64_t H, int64_t I, const void* weights, int w_dtype,
-              int64_t w_stride, int out_dtype, const int32_t* dest, int64_t dest_stride, void* const* peer_out,
-              int n_peers, int64_t peer_rows, void* stream) {
-    int rc = fg_moe_grouped_gemm_fp8(ws.act, ws.a1, w1, ws.a1s, s1, nullptr, 0, 1, ws.sorted_ids, ws.expert_ids,
-                                     ws.post_pad, ws.rows, n_in, num_experts, 2 * I, H, H, I, TILE_ROWS, FG_SCALE_BLOCK,
-                                     1, /*fuse_silu=*/1, /*scatter=*/0, /*mul_weight=*/0, out_dtype, stream);
+// One layer's experts on tokens of this GPU.
+struct Experts {
+    int mode;
+    const void* hidden;
+    int dtype;
+    const void* topk_w;
+    int topk_w_dtype;
+    int64_t T;
+    int topk;
+    const void *w1, *w2;
+    const float *s1, *s2, *a1_scale, *a2_scale;
+    int local_experts;
+    int64_t H, I;
+    bool gathered;
+};
+
+// The line between the two row orders (see the head of this file).
+bool use_gather(int64_t slots, int num_experts) { return slots <= 32 * (int64_t)num_experts; }
+
+// Rows of one GEMM's input in the operand type of the mode; *scale is where their scales are.
+int quantise(int mode, const void* x, int dtype, uint8_t* q, float* s, float* scalars, const float* given, int64_t src_rows,
+             int64_t rows, int64_t K, const int32_t* index, int div, int64_t limit, const int32_t* n_rows_dev, const float** scale,
+             cudaStream_t st) {
+    *scale = s;
+    const int kind = mode == FG_EXPERTS_BLOCK_FP8 ? FG_QUANT_GROUP128 : mode == FG_EXPERTS_CHANNEL_FP8 ? FG_QUANT_TOKEN
+                     : mode == FG_EXPERTS_CHANNEL_INT8 ? FG_QUANT_INT8 : FG_QUANT_TENSOR;
+    const float* tensor = given;
+    if (kind == FG_QUANT_TENSOR) {
+        *scale = given ? given : scalars + 1;
+        if (!given) {  // scalars[0]: amax, scalars[1]: the scale derived from it
+            FG_CUDA(cudaMemsetAsync(scalars, 0, 4, st));
+            const int rc = fg_abs_max(x, dtype, src_rows, K, K, index && div == 0 ? n_rows_dev : nullptr, scalars, st);
+            if (rc != FG_OK) return rc;
+            tensor = scalars;
+        }
+    }
+    return fg_quant_rows(kind, x, dtype, q, s, tensor, given ? nullptr : scalars + 1, rows, K, index, div, (int32_t)limit,
+                         n_rows_dev, st);
+}
+
+// align has run: quantise -> GEMM1 -> quantise -> GEMM2 into y (route-slot order).
+int run_experts(const Experts& e, const Workspace& ws, void* y, cudaStream_t st) {
+    const int64_t slots = e.T * e.topk;
+    const bool unit = e.mode == FG_EXPERTS_16BIT, plain = unit || e.mode == FG_EXPERTS_16BIT_SCALED;
+    const bool block = e.mode == FG_EXPERTS_BLOCK_FP8, tensor = e.mode == FG_EXPERTS_TENSOR_FP8;
+    const int esz = e.dtype == FG_DTYPE_F32 ? 4 : 2;
+    const void *a1 = ws.a1, *a2 = ws.a2;
+    const float *a1s = ws.a1s, *a2s = ws.a2s, *s1 = e.s1, *s2 = e.s2;
+    int rc = FG_OK;
+    if (plain) {
+        // unquantised activations: unit scales, per expert or (with scaled weights) per row
+        float* ones = unit ? ws.scalars : ws.a1s;
+        rc = fg_fill_ones(ones, unit ? e.local_experts : ws.rows, st);
+        if (rc != FG_OK) return rc;
+        a1s = a2s = ones;
+        if (unit) s1 = s2 = ones;
+        a2 = ws.act;
+        if (e.gathered) a1 = e.hidden;
+        else rc = fg_gather_rows_fp8(e.hidden, nullptr, ws.a1, nullptr, ws.rows, 2 * e.H, 0, 2 * e.H, 1, ws.sorted_ids, e.topk,
+                                 (int32_t)slots, ws.post_pad, st);
+    } else if (e.gathered) {
+        rc = quantise(e.mode, e.hidden, e.dtype, ws.a1, ws.a1s, ws.scalars, e.a1_scale, e.T, e.T, e.H, nullptr, 1, 0, nullptr, &a1s, st);
+    } else {
+        // Each token is quantised once and its row copied to its top-k places; with one or two places
+        // quantising while copying moves no more bytes and saves the launch.  The token rows borrow the
+        // room of GEMM1's output, which is first written after the copy has finished.
+        const int64_t s_cols = block ? e.H / 128 : 1, tok_q_bytes = align_up(e.T * e.H, 256);
+        if (e.topk > 2 && !tensor && tok_q_bytes + 4 * e.T * s_cols <= ws.rows * e.I * esz) {
+            uint8_t* tok_q = ws.act;
+            float* tok_s = reinterpret_cast<float*>(ws.act + tok_q_bytes);
+            rc = quantise(e.mode, e.hidden, e.dtype, tok_q, tok_s, ws.scalars, nullptr, e.T, e.T, e.H, nullptr, 1, 0, nullptr, &a1s, st);
+            if (rc != FG_OK) return rc;
+            a1s = ws.a1s;
+            rc = fg_gather_rows_fp8(tok_q, tok_s, ws.a1, ws.a1s, ws.rows, e.H, s_cols, e.H, s_cols, ws.sorted_ids, e.topk, (int32_t)slots,
+                                ws.post_pad, st);
+        } else {
+            rc = quantise(e.mode, e.hidden, e.dtype, ws.a1, ws.a1s, ws.scalars, e.a1_scale, e.T, ws.rows, e.H, ws.sorted_ids, e.topk,
+                          slots, ws.post_pad, &a1s, st);
+        }
+    }
     if (rc != FG_OK) return rc;
-    rc = fg_per_token_group_quant_fp8_gather(ws.act, out_dtype, ws.a2, ws.a2s, ws.rows, I, 128, I, I, nullptr, 1, 0,
-                                             ws.post_pad, stream);
+
+    FgGroupedGemm g{};
+    g.sorted_ids = ws.sorted_ids; g.expert_ids = ws.expert_ids; g.num_post_pad = ws.post_pad; g.max_rows = ws.rows;
+    g.numel = slots; g.num_experts = e.local_experts; g.block_rows = TILE_ROWS; g.out_dtype = e.dtype;
+    g.operand = plain ? (e.dtype == FG_DTYPE_BF16 ? 2 : 3) : e.mode == FG_EXPERTS_CHANNEL_INT8 ? 1 : 0;
+    g.scale_mode = block ? FG_SCALE_BLOCK : (unit || tensor) ? FG_SCALE_SCALAR : FG_SCALE_VECTOR;
+    g.c = ws.act; g.a = a1; g.w = e.w1; g.a_scale = a1s; g.w_scale = s1; g.a_rows = e.T; g.gather_div = e.gathered ? e.topk : 0;
+    g.N = 2 * e.I; g.K = e.H; g.ld_a = e.H; g.ld_as = e.H / 128; g.ld_c = e.I; g.fuse_silu = 1; g.scatter = e.gathered;
+    rc = fg_grouped_gemm(g, st);
     if (rc != FG_OK) return rc;
-    return fg_moe_grouped_gemm_fp8_peer(y, ws.a2, w2, ws.a2s, s2, weights, w_dtype, w_stride, ws.sorted_ids,
-                                        ws.expert_ids, ws.post_pad, ws.rows, n_in, num_experts, H, I, I, H, TILE_ROWS,
-                                        FG_SCALE_BLOCK, 1, /*fuse_silu=*/0, /*scatter=*/1, /*mul_weight=*/1, out_dtype,
-                                        dest, dest_stride, peer_out, n_peers, peer_rows, stream);
+    if (!plain) {
+        if (e.gathered) rc = quantise(e.mode, ws.act, e.dtype, ws.a2, ws.a2s, ws.scalars + 2, e.a2_scale, slots, slots, e.I, nullptr, 1,
+                                      0, nullptr, &a2s, st);
+        else rc = quantise(e.mode, ws.act, e.dtype, ws.a2, ws.a2s, ws.scalars + 2, e.a2_scale, ws.rows, ws.rows, e.I, ws.sorted_ids, 0,
+                           slots, ws.post_pad, &a2s, st);
+        if (rc != FG_OK) return rc;
+    }
+    g.c = y; g.a = a2; g.w = e.w2; g.a_scale = a2s; g.w_scale = s2; g.a_rows = slots; g.gather_div = e.gathered ? 1 : 0;
+    g.N = e.H; g.K = e.I; g.ld_a = e.I; g.ld_as = e.I / 128; g.ld_c = e.H; g.fuse_silu = 0; g.scatter = 1; g.mul_weight = 1;
+    g.topk_w = e.topk_w; g.topk_w_dtype = e.topk_w_dtype; g.topk_w_stride = 1;
+    return fg_grouped_gemm(g, st);
 }
 
 // Device address of g_routed_scratch on the current device, looked up once per device.
@@ -102,36 +210,12 @@ int builtin_scratch(void** out) {
 
 namespace {
 
-// Scratch of fg_scaled_grouped_mm_fp8.
-struct GroupedMmWorkspace {
-    int32_t* group_ids;
-    int32_t* sorted_ids;
-    int32_t* expert_ids;
-    int32_t* post_pad;
-    uint8_t* a_sorted;
-    float* sa_sorted;
-    int64_t max_pad, n_blocks, rows, bytes;
-};
-
-GroupedMmWorkspace carve_grouped_mm(void* base, int64_t m_total, int num_groups, int64_t K) {
-    GroupedMmWorkspace w{};
-    w.max_pad = m_total + (int64_t)num_groups * (TILE_ROWS - 1);
-    w.n_blocks = fg_cdiv(w.max_pad, TILE_ROWS);
-    w.rows = w.max_pad / TILE_ROWS * TILE_ROWS;
-    uint8_t* p = reinterpret_cast<uint8_t*>(base);
-    int64_t off = 0;
-    auto take = [&](int64_t bytes) {
-        uint8_t* r = p ? p + off : nullptr;
-        off += align_up(bytes, 256);
-        return r;
-    };
-    w.group_ids = (int32_t*)take(4 * m_total);
-    w.sorted_ids = (int32_t*)take(4 * w.max_pad);
-    w.expert_ids = (int32_t*)take(4 * w.n_blocks);
-    w.post_pad = (int32_t*)take(256);
-    w.a_sorted = take(w.rows * K);
-    w.sa_sorted = (float*)take(4 * w.rows);
-    w.bytes = off;
+// Scratch of fg_scaled_grouped_mm_fp8: the alignment tables only.
+Workspace carve_grouped_mm(void* base, int64_t m_total, int num_groups) {
+    Workspace w{};
+    Carver c{reinterpret_cast<uint8_t*>(base), 0};
+    carve_tables(c, w, m_total, num_groups);
+    w.bytes = c.off;
     return w;
 }
 
@@ -141,7 +225,7 @@ extern "C" {
 
 int64_t fg_scaled_grouped_mm_workspace_bytes(int64_t m_total, int num_groups, int64_t K) {
     if (m_total < 0 || num_groups <= 0 || K <= 0) return -1;
-    return carve_grouped_mm(nullptr, m_total, num_groups, K).bytes;
+    return carve_grouped_mm(nullptr, m_total, num_groups).bytes;
 }
 
 int fg_scaled_grouped_mm_fp8(void* c, const void* a, const void* b, const float* scale_a, const float* scale_b,
@@ -154,20 +238,21 @@ int fg_scaled_grouped_mm_fp8(void* c, const void* a, const void* b, const float*
     if (m_total == 0) return FG_OK;
     FG_REQUIRE(c && a && b && scale_a && scale_b && offs && workspace, FG_ERR_INVALID_ARGUMENT, "null pointer");
     FG_REQUIRE((uintptr_t)workspace % 256 == 0, FG_ERR_INVALID_ARGUMENT, "workspace must be 256-byte aligned");
-    const GroupedMmWorkspace ws = carve_grouped_mm(workspace, m_total, num_groups, K);
+    FG_REQUIRE(ld_a % 16 == 0 && (uintptr_t)a % 16 == 0, FG_ERR_UNSUPPORTED, "a must have 16-byte aligned rows");
+    const Workspace ws = carve_grouped_mm(workspace, m_total, num_groups);
     FG_REQUIRE(workspace_bytes >= ws.bytes, FG_ERR_INVALID_ARGUMENT, "workspace holds %lld bytes, needs %lld",
                (long long)workspace_bytes, (long long)ws.bytes);
-    int rc = fg_group_ids_from_offsets(offs, num_groups, m_total, ws.group_ids, stream);
+    cudaStream_t st = (cudaStream_t)stream;
+    int rc = fg_group_tiles(offs, num_groups, m_total, TILE_ROWS, ws.sorted_ids, ws.max_pad, ws.expert_ids, ws.n_blocks,
+                            ws.post_pad, st);
     if (rc != FG_OK) return rc;
-    rc = fg_moe_align_block_size(ws.group_ids, 0, m_total, num_groups, TILE_ROWS, nullptr, 0, ws.sorted_ids, ws.max_pad,
-                                 ws.expert_ids, ws.n_blocks, ws.post_pad, stream);
-    if (rc != FG_OK) return rc;
-    rc = fg_gather_rows_fp8(a, scale_a, ws.a_sorted, ws.sa_sorted, ws.rows, K, 1, ld_a, 1, ws.sorted_ids, 1,
-                            (int32_t)m_total, ws.post_pad, stream);
-    if (rc != FG_OK) return rc;
-    return fg_grouped_gemm_fp8_bias(c, ws.a_sorted, b, ws.sa_sorted, scale_b, bias, bias_stride_g, ws.sorted_ids,
-                                    ws.expert_ids, ws.post_pad, ws.rows, m_total, num_groups, N, K, K, ld_c, out_dtype,
-                                    stream);
+    FgGroupedGemm g{};
+    g.sorted_ids = ws.sorted_ids; g.expert_ids = ws.expert_ids; g.num_post_pad = ws.post_pad; g.max_rows = ws.rows;
+    g.numel = m_total; g.num_experts = num_groups; g.block_rows = TILE_ROWS; g.scale_mode = FG_SCALE_VECTOR; g.out_dtype = out_dtype;
+    g.c = c; g.a = a; g.w = b; g.a_scale = scale_a; g.w_scale = scale_b; g.bias = bias; g.bias_stride = bias_stride_g;
+    // few rows per group: only they are fetched; otherwise a block is one box from its first row
+    g.a_rows = m_total; g.gather_div = 1; g.a_contiguous = !use_gather(m_total, num_groups); g.N = N; g.K = K; g.ld_a = ld_a; g.ld_c = ld_c; g.scatter = 1;
+    return fg_grouped_gemm(g, st);
 }
 
 int64_t fg_moe_routed_workspace_bytes(int64_t n_rows_in, int num_experts, int64_t H, int64_t I) {
@@ -192,27 +277,9 @@ int fg_moe_routed_block_fp8_local(void* y, const void* hidden, int hidden_dtype,
     rc = fg_moe_align_block_size(topk_ids, ids_are_i64, n_in, num_experts, TILE_ROWS, nullptr, 0, ws.sorted_ids,
                                  ws.max_pad, ws.expert_ids, ws.n_blocks, ws.post_pad, stream);
     if (rc != FG_OK) return rc;
-    // Every token is quantised once (as the reference does before its gathering GEMM) and its FP8 row
-    // and scales are then copied to each of its top-k places in expert order: quantising while gathering
-    // would read and quantise every token top-k times.  The token buffer borrows the room of GEMM1's
-    // output, which is first written after the copy has finished.  Bits are the same either way.
-    const int64_t s_cols = H / 128;
-    const int64_t tok_q_bytes = align_up(T * H, 256);
-    if (topk > 1 && tok_q_bytes + 4 * T * s_cols <= ws.rows * I * 2) {
-        uint8_t* tok_q = ws.act;
-        float* tok_s = reinterpret_cast<float*>(ws.act + tok_q_bytes);
-        rc = fg_per_token_group_quant_fp8(hidden, hidden_dtype, tok_q, tok_s, T, H, 128, H, H, s_cols, 1, 1e-10f, 0,
-                                          stream);
-        if (rc != FG_OK) return rc;
-        rc = fg_gather_rows_fp8(tok_q, tok_s, ws.a1, ws.a1s, ws.rows, H, s_cols, H, s_cols, ws.sorted_ids, topk,
-                                (int32_t)n_in, ws.post_pad, stream);
-    } else {
-        rc = fg_per_token_group_quant_fp8_gather(hidden, hidden_dtype, ws.a1, ws.a1s, ws.rows, H, 128, H, H,
-                                                 ws.sorted_ids, topk, (int32_t)n_in, ws.post_pad, stream);
-    }
-    if (rc != FG_OK) return rc;
-    return run_gemms(y, ws, n_in, w1, w2, s1, s2, num_experts, H, I, topk_w, topk_w_dtype, 1, hidden_dtype, nullptr, 0,
-                     nullptr, 0, 0, stream);
+    const Experts e{FG_EXPERTS_BLOCK_FP8, hidden, hidden_dtype, topk_w, topk_w_dtype, T, topk, w1, w2, s1, s2, nullptr, nullptr,
+                    num_experts, H, I, use_gather(n_in, num_experts)};
+    return run_experts(e, ws, y, (cudaStream_t)stream);
 }
 
 int fg_moe_routed_block_fp8_packed(void* y, const void* rows, int64_t R, int64_t row_bytes, const void* w1,
@@ -240,12 +307,29 @@ int fg_moe_routed_block_fp8_packed(void* y, const void* rows, int64_t R, int64_t
                                          ws.expert_ids, ws.n_blocks, ws.post_pad, row_bytes / 4, 1, nullptr,
                                          n_rows_dev, region_rows, region_counts, region_stride, stream);
     if (rc != FG_OK) return rc;
-    rc = fg_gather_rows_fp8(base, reinterpret_cast<const float*>(base + H), ws.a1, ws.a1s, ws.rows, H, s_cols,
-                            row_bytes, row_bytes / 4, ws.sorted_ids, 1, (int32_t)R, ws.post_pad, stream);
+    cudaStream_t st = (cudaStream_t)stream;
+    rc = fg_gather_rows_fp8(base, reinterpret_cast<const float*>(base + H), ws.a1, ws.a1s, ws.rows, H, s_cols, row_bytes, row_bytes / 4,
+                        ws.sorted_ids, 1, (int32_t)R, ws.post_pad, st);
     if (rc != FG_OK) return rc;
-    const int32_t* dest = reinterpret_cast<const int32_t*>(base + H + 4 * s_cols + 8);
-    return run_gemms(y, ws, R, w1, w2, s1, s2, num_experts, H, I, wts, FG_DTYPE_F32, row_bytes / 4, out_dtype,
-                     n_peers > 0 ? dest : nullptr, row_bytes / 4, peer_out, n_peers, peer_rows, stream);
+    FgGroupedGemm g{};
+    g.sorted_ids = ws.sorted_ids; g.expert_ids = ws.expert_ids; g.num_post_pad = ws.post_pad; g.max_rows = ws.rows;
+    g.numel = R; g.num_experts = num_experts; g.block_rows = TILE_ROWS; g.scale_mode = FG_SCALE_BLOCK; g.out_dtype = out_dtype;
+    g.c = ws.act; g.a = ws.a1; g.w = w1; g.a_scale = ws.a1s; g.w_scale = s1;
+    g.N = 2 * I; g.K = H; g.ld_a = H; g.ld_as = s_cols; g.ld_c = I; g.fuse_silu = 1;
+    rc = fg_grouped_gemm(g, st);
+    if (rc != FG_OK) return rc;
+    rc = fg_quant_rows(FG_QUANT_GROUP128, ws.act, out_dtype, ws.a2, ws.a2s, nullptr, nullptr, ws.rows, I, ws.sorted_ids, 0, (int32_t)R,
+                       ws.post_pad, st);
+    if (rc != FG_OK) return rc;
+    g.c = y; g.a = ws.a2; g.w = w2; g.a_scale = ws.a2s; g.w_scale = s2;
+    g.N = H; g.K = I; g.ld_a = I; g.ld_as = I / 128; g.ld_c = H; g.fuse_silu = 0; g.scatter = 1; g.mul_weight = 1;
+    g.topk_w = wts; g.topk_w_dtype = FG_DTYPE_F32; g.topk_w_stride = row_bytes / 4;
+    if (n_peers > 0) {
+        g.dest = reinterpret_cast<const int32_t*>(base + H + 4 * s_cols + 8);
+        g.dest_stride = row_bytes / 4;
+        g.peer_out = peer_out; g.n_peers = n_peers; g.peer_rows = peer_rows;
+    }
+    return fg_grouped_gemm(g, st);
 }
 
 int fg_moe_routed_block_fp8_local_noalloc(void* y, const void* hidden, int hidden_dtype, const void* topk_ids,
@@ -265,6 +349,57 @@ int fg_moe_routed_block_fp8_local_noalloc(void* y, const void* hidden, int hidde
     if (rc != FG_OK) return rc;
     return fg_moe_routed_block_fp8_local(y, hidden, hidden_dtype, topk_ids, ids_are_i64, topk_w, topk_w_dtype, T, topk,
                                          w1, w2, s1, s2, num_experts, H, I, scratch, FG_NOALLOC_SCRATCH_BYTES, stream);
+}
+
+// Workspace of fg_fused_experts in one mode.
+static Workspace carve_experts(void* base, int mode, int64_t T, int topk, int num_experts, int64_t H, int64_t I, int esz) {
+    Workspace w{};
+    Carver c{reinterpret_cast<uint8_t*>(base), 0};
+    const int64_t slots = T * topk;
+    const bool gathered = use_gather(slots, num_experts), plain = mode == FG_EXPERTS_16BIT || mode == FG_EXPERTS_16BIT_SCALED;
+    const int64_t cols1 = mode == FG_EXPERTS_BLOCK_FP8 ? H / 128 : 1, cols2 = mode == FG_EXPERTS_BLOCK_FP8 ? I / 128 : 1;
+    carve_tables(c, w, slots, num_experts);
+    const int64_t rows1 = gathered ? T : w.rows, rows2 = gathered ? slots : w.rows;
+    w.scalars = (float*)c.take(4 * (num_experts > 64 ? num_experts : 64));
+    w.a1 = c.take(plain ? (gathered ? 0 : rows1 * H * 2) : rows1 * H);
+    w.a1s = (float*)c.take(4 * (plain ? w.rows : rows1 * cols1));
+    w.act = c.take(rows2 * I * esz);
+    w.a2 = c.take(plain ? 0 : rows2 * I);
+    w.a2s = (float*)c.take(4 * rows2 * cols2);
+    w.routed = c.take(slots * H * esz);
+    w.bytes = c.off;
+    return w;
+}
+
+int64_t fg_fused_experts_workspace_bytes(int mode, int64_t T, int topk, int num_experts, int64_t H, int64_t I,
+                                         int hidden_dtype) {
+    if (T < 0 || topk <= 0 || num_experts <= 0 || H <= 0 || I <= 0) return -1;
+    return carve_experts(nullptr, mode, T, topk, num_experts, H, I, hidden_dtype == FG_DTYPE_F32 ? 4 : 2).bytes;
+}
+
+int fg_fused_experts(void* out, const void* hidden, int hidden_dtype, const void* topk_ids, int ids_are_i64, const void* topk_w,
+                     int topk_w_dtype, int64_t T, int topk, const void* w1, const void* w2, const float* s1, const float* s2,
+                     const float* a1_scale, const float* a2_scale, int mode, int num_experts, int local_experts,
+                     const int32_t* expert_map, int expert_map_len, int64_t H, int64_t I, const void* addend, void* workspace,
+                     int64_t workspace_bytes, void* stream) {
+    FG_REQUIRE(T >= 0 && topk > 0 && num_experts > 0 && local_experts > 0 && H > 0 && I > 0, FG_ERR_INVALID_ARGUMENT, "bad sizes");
+    FG_REQUIRE(mode >= FG_EXPERTS_BLOCK_FP8 && mode <= FG_EXPERTS_16BIT_SCALED, FG_ERR_INVALID_ARGUMENT, "bad mode %d", mode);
+    if (T == 0) return FG_OK;
+    FG_REQUIRE(out && hidden && topk_ids && topk_w && w1 && w2 && workspace && (mode == FG_EXPERTS_16BIT || (s1 && s2)),
+               FG_ERR_INVALID_ARGUMENT, "null pointer");
+    FG_REQUIRE(T * topk < (1ll << 31), FG_ERR_UNSUPPORTED, "too many route slots");
+    FG_REQUIRE(local_experts <= num_experts, FG_ERR_INVALID_ARGUMENT, "more local experts than experts");
+    const Workspace ws = carve_experts(workspace, mode, T, topk, num_experts, H, I, hidden_dtype == FG_DTYPE_F32 ? 4 : 2);
+    FG_REQUIRE((uintptr_t)workspace % 256 == 0 && workspace_bytes >= ws.bytes, FG_ERR_INVALID_ARGUMENT,
+               "workspace holds %lld bytes, needs %lld (256-byte aligned)", (long long)workspace_bytes, (long long)ws.bytes);
+    int rc = fg_moe_align_block_size(topk_ids, ids_are_i64, T * topk, num_experts, TILE_ROWS, expert_map, expert_map_len,
+                                     ws.sorted_ids, ws.max_pad, ws.expert_ids, ws.n_blocks, ws.post_pad, stream);
+    if (rc != FG_OK) return rc;
+    const Experts e{mode, hidden, hidden_dtype, topk_w, topk_w_dtype, T, topk, w1, w2, s1, s2, a1_scale, a2_scale,
+                    local_experts, H, I, use_gather(T * topk, num_experts)};
+    rc = run_experts(e, ws, ws.routed, (cudaStream_t)stream);
+    if (rc != FG_OK) return rc;
+    return fg_moe_sum_indexed(ws.routed, out, T, topk, H, hidden_dtype, nullptr, addend, stream);
 }
 
 }  // extern "C"

@@ -28,7 +28,7 @@ struct QuantArgs {
     float eps;
     int pow2;
     const int32_t* row_index;  // nullable gather
-    int32_t index_div;
+    int32_t index_div;         // 0: row r reads row r, the index only tells padding rows
     int32_t index_limit;
     const int32_t* n_rows_dev;  // nullable
     // Optional per-row trailer of the expert-parallel dispatch format (see fg_ep_pack_rows_fp8):
@@ -127,7 +127,8 @@ __device__ __forceinline__ int64_t resolve_rows(const QuantArgs& a) {
 __device__ __forceinline__ int64_t source_row(const QuantArgs& a, int64_t r) {
     if (!a.row_index) return r;
     int32_t idx = a.row_index[r];
-    return (idx >= 0 && idx < a.index_limit) ? (int64_t)(idx / a.index_div) : -1;
+    if (idx < 0 || idx >= a.index_limit) return -1;
+    return a.index_div > 0 ? (int64_t)(idx / a.index_div) : r;
 }
 
 // ---- small groups: a team of TPG lanes owns one group of TPG*8*VPT elements -------------
@@ -858,3 +859,23 @@ int fg_per_token_quant_fp8(const void* x, int x_dtype, void* q, float* s, int64_
 }
 
 }  // extern "C"
+
+int fg_quant_rows(int kind, const void* x, int x_dtype, void* q, float* s, const float* tensor_scale, float* scale_out, int64_t rows,
+                  int64_t K, const int32_t* row_index, int32_t index_div, int32_t index_limit, const int32_t* n_rows_dev,
+                  cudaStream_t st) {
+    QuantArgs a{};
+    a.x = x; a.q = (uint8_t*)q; a.s = s; a.rows = rows; a.K = K; a.ld_x = K; a.ld_q = K;
+    a.group = kind == FG_QUANT_GROUP128 ? 128 : (int)K;
+    a.s_row_stride = kind == FG_QUANT_GROUP128 ? K / 128 : 1; a.s_col_stride = 1; a.eps = 1e-10f;
+    a.row_index = row_index; a.index_div = index_div; a.index_limit = index_limit; a.n_rows_dev = n_rows_dev;
+    a.tensor_scale = tensor_scale; a.tensor_scale_out = scale_out;
+    if (kind == FG_QUANT_TENSOR) a.s = const_cast<float*>(tensor_scale);
+    const int rc = check_common(a, x_dtype);
+    if (rc != FG_OK || rows == 0) return rc;
+    switch (kind) {
+        case FG_QUANT_GROUP128: return launch_quant<QM_GROUP>(x_dtype, a, st);
+        case FG_QUANT_TOKEN: return launch_rows<QM_TOKEN>(x_dtype, a, st);
+        case FG_QUANT_INT8: return launch_rows<QM_INT8_TOKEN>(x_dtype, a, st);
+        default: return scale_out ? launch_rows<QM_TENSOR_DYNAMIC>(x_dtype, a, st) : launch_rows<QM_TENSOR_STATIC>(x_dtype, a, st);
+    }
+}

@@ -5,8 +5,8 @@ Mirrors the FP8 path of src/flag_gems/fused/fused_moe.py of the reference:
 ``fused_experts_impl`` (:1821-2185), ``inplace_fused_experts`` / ``outplace_fused_experts``
 (:2188-2290), ``_fp8_quantize`` / ``moe_kernel_quantize_input`` (:629-698, :749-773),
 ``MoEActivation`` (:538-577).  The two grouped GEMMs are ``fg_moe_grouped_gemm_fp8``
-(tcgen05); rows are first gathered into expert-sorted padded order while they are
-quantised, so the GEMMs read their A operand with plain TMA boxes.
+(tcgen05); a layer runs as one native call (``fg_fused_experts``), whose GEMMs fetch their rows
+through ``sorted_ids``.
 
 Implemented: the FP8 w8a8 modes (block 128x128, per-token x per-channel, per-tensor) and int8
 w8a8 with per-token x per-channel scales (tcgen05 kind::i8, int32 accumulation); the weight-only
@@ -20,9 +20,7 @@ from typing import Optional
 import torch
 
 from .. import _cabi
-from .moe_align_block_size import ceil_div, moe_align_block_size
-from .moe_sum import moe_sum
-from .silu_and_mul import silu_and_mul_out
+from .moe_align_block_size import ceil_div
 
 logger = logging.getLogger(__name__.replace("flaggems_b200", "flag_gems", 1))
 
@@ -244,14 +242,13 @@ def _fused_experts_16bit(hidden_states, w1, w2, topk_weights, topk_ids, inplace,
     dtype = hidden_states.dtype
     if dtype not in (torch.bfloat16, torch.float16):
         raise NotImplementedError(f"16-bit expert GEMMs take bf16 or fp16 activations, got {dtype}")
-    num_tokens, hidden = hidden_states.shape
+    hidden = hidden_states.size(1)
     e, n, _ = w1.shape
     k_out = w2.size(1)
     inter = n // 2
     assert w2.size(2) == inter, "w2 inner size must be half of w1's output size"
     if hidden % 8 or inter % 8:
         raise NotImplementedError("hidden and intermediate sizes must be multiples of 8")
-    dev = hidden_states.device
     if weight_only:
         if w1.dtype != torch.int8 or w2.dtype != torch.int8:
             raise NotImplementedError("weight-only experts are int8 tensors (int4 values in int8 containers)")
@@ -260,43 +257,30 @@ def _fused_experts_16bit(hidden_states, w1, w2, topk_weights, topk_ids, inplace,
         w2s = w2_scale.float().reshape(e, -1).contiguous()
         assert w1s.shape == (e, n) and w2s.shape == (e, k_out), "per-channel scales must be [E, N]"
         w1, w2 = w1.to(dtype), w2.to(dtype)  # exact: |v| <= 128
-        scale_mode = _cabi.SCALE_VECTOR
+        mode = _cabi.EXPERTS_16BIT_SCALED
     else:
         if w1.dtype != dtype or w2.dtype != dtype:
             raise NotImplementedError(f"unquantised expert weights must have the activation type {dtype}")
-        w1s = w2s = torch.ones(e, dtype=torch.float32, device=dev)
-        scale_mode = _cabi.SCALE_SCALAR
-    if global_num_experts == -1:
-        global_num_experts = e
-    top_k = topk_ids.size(1)
+        w1s = w2s = None
+        mode = _cabi.EXPERTS_16BIT
+    return _run_experts(hidden_states, w1, w2, topk_weights, topk_ids, inplace, mode, w1s, w2s, None, None,
+                        e if global_num_experts == -1 else global_num_experts, expert_map)
+
+
+def _run_experts(hidden_states, w1, w2, topk_weights, topk_ids, inplace, mode, w1s, w2s, a1_scale, a2_scale,
+                 global_num_experts, expert_map):
+    """The device work of a layer (``fg_fused_experts``) in chunks of tokens."""
     out = hidden_states if inplace else torch.empty_like(hidden_states)
-    if num_tokens == 0:
+    if hidden_states.shape[0] == 0:
         return out
+    assert w2.size(1) == out.size(1), "output shape mismatch"
     tw = topk_weights if topk_weights.dtype in _cabi.DTYPE_CODE else topk_weights.float()
-    tw = tw.contiguous()
-    with _cabi.device_guard(hidden_states):
-        for begin in range(0, num_tokens, _CHUNK_SIZE):
-            end = min(begin + _CHUNK_SIZE, num_tokens)
-            h = hidden_states[begin:end]
-            ids = topk_ids[begin:end]
-            w = tw[begin:end].reshape(-1)
-            t = end - begin
-            numel = t * top_k
-            sorted_ids, expert_ids, post_pad = moe_align_block_size(ids, _TILE_ROWS, global_num_experts, expert_map)
-            rows = sorted_ids.numel() // _TILE_ROWS * _TILE_ROWS
-            # rows into expert order: a byte copy of the 16-bit rows (zeros for padding rows)
-            a1 = torch.empty((rows, hidden), dtype=dtype, device=dev)
-            _cabi.check(_cabi.lib().fg_gather_rows_fp8(
-                _cabi.ptr(h), None, _cabi.ptr(a1), None, rows, 2 * hidden, 0, 2 * h.stride(0), 1,
-                _cabi.ptr(sorted_ids), top_k, numel, _cabi.ptr(post_pad), _cabi.stream_ptr(dev)))
-            ones = torch.ones(rows if scale_mode == _cabi.SCALE_VECTOR else 1, dtype=torch.float32, device=dev)
-            act = torch.empty((rows, inter), dtype=dtype, device=dev)
-            _grouped_gemm(act, a1, w1, ones, w1s, None, sorted_ids, expert_ids, post_pad, numel, scale_mode,
-                          fuse_silu=True, scatter=False, mul_weight=False)
-            routed = torch.empty((t, top_k, k_out), dtype=dtype, device=dev)
-            _grouped_gemm(routed, act, w2, ones, w2s, w, sorted_ids, expert_ids, post_pad, numel, scale_mode,
-                          fuse_silu=False, scatter=True, mul_weight=True)
-            moe_sum(routed, out[begin:end])
+    if topk_ids.dtype not in (torch.int32, torch.int64):
+        raise NotImplementedError(f"topk_ids must be int32 or int64, got {topk_ids.dtype}")
+    emap = None if expert_map is None else expert_map.to(torch.int32).contiguous()
+    done = _cabi.host.fused_experts(hidden_states, w1, w2, tw.contiguous(), topk_ids.contiguous(), out, mode, w1s, w2s,
+                                    a1_scale, a2_scale, global_num_experts, emap, _CHUNK_SIZE)
+    assert done is not None
     return out
 
 
@@ -362,79 +346,40 @@ def fused_experts_impl(
     if w1.dtype != w_dtype or w2.dtype != w_dtype:
         raise NotImplementedError(f"expert weights must be {w_dtype}")
 
-    num_tokens, hidden = hidden_states.shape
+    hidden = hidden_states.size(1)
     e, n, _ = w1.shape
     k_out = w2.size(1)
     inter = n // 2
     assert w2.size(2) == inter, "w2 inner size must be half of w1's output size"
     if global_num_experts == -1:
         global_num_experts = e
-    top_k = topk_ids.size(1)
-    dtype = hidden_states.dtype
 
     if block_shape is not None:
         assert len(block_shape) == 2
         if list(block_shape) != [128, 128]:
             raise NotImplementedError(f"block_shape {block_shape}: only [128, 128] is implemented")
         assert hidden % 128 == 0 and inter % 128 == 0, "block-FP8 needs hidden and intermediate sizes divisible by 128"
-        scale_mode = _cabi.SCALE_BLOCK
+        mode = _cabi.EXPERTS_BLOCK_FP8
         w1s = w1_scale.float().contiguous()
         w2s = w2_scale.float().contiguous()
         assert w1s.shape == (e, (n + 127) // 128, hidden // 128), f"w1_scale shape {tuple(w1s.shape)}"
         assert w2s.shape == (e, (k_out + 127) // 128, inter // 128), f"w2_scale shape {tuple(w2s.shape)}"
     elif per_channel_quant:
-        scale_mode = _cabi.SCALE_VECTOR
+        mode = _cabi.EXPERTS_CHANNEL_INT8 if use_int8_w8a8 else _cabi.EXPERTS_CHANNEL_FP8
         w1s = w1_scale.float().reshape(e, -1).contiguous()
         w2s = w2_scale.float().reshape(e, -1).contiguous()
         assert w1s.shape == (e, n) and w2s.shape == (e, k_out), "per-channel scales must be [E, N]"
     else:
-        scale_mode = _cabi.SCALE_SCALAR  # one scale per expert, one per activation tensor
+        mode = _cabi.EXPERTS_TENSOR_FP8  # one scale per expert, one per activation tensor
         w1s = w1_scale.float().reshape(-1).contiguous()
         w2s = w2_scale.float().reshape(-1).contiguous()
         assert w1s.numel() == e and w2s.numel() == e, "per-tensor weight scales must hold one value per expert"
 
-    out = hidden_states if inplace else torch.empty_like(hidden_states)
-    if num_tokens == 0:
-        return out
-    tw = topk_weights if topk_weights.dtype in _cabi.DTYPE_CODE else topk_weights.float()
-    tw = tw.contiguous()
+    def scalar(scale):
+        return None if scale is None else scale.float().reshape(-1)[:1].contiguous()
 
-    with _cabi.device_guard(hidden_states):
-        for begin in range(0, num_tokens, _CHUNK_SIZE):
-            end = min(begin + _CHUNK_SIZE, num_tokens)
-            h = hidden_states[begin:end]
-            ids = topk_ids[begin:end]
-            w = tw[begin:end].reshape(-1)
-            t = end - begin
-            numel = t * top_k
-
-            sorted_ids, expert_ids, post_pad = moe_align_block_size(ids, _TILE_ROWS, global_num_experts, expert_map)
-            rows = sorted_ids.numel() // _TILE_ROWS * _TILE_ROWS
-
-            if scale_mode == _cabi.SCALE_BLOCK:
-                if top_k > 1:
-                    a1, a1s = _group_quant_once_then_gather(h, 128, sorted_ids, top_k, numel, post_pad, rows)
-                else:
-                    a1, a1s = _group_quant(h, 128, sorted_ids, top_k, numel, post_pad, rows)
-            elif scale_mode == _cabi.SCALE_VECTOR:
-                quant_rows = _per_token_quant_int8 if use_int8_w8a8 else _per_token_quant
-                a1, a1s = quant_rows(h, sorted_ids, top_k, numel, post_pad, rows)
-            else:
-                a1, a1s = _per_tensor_quant(h, a1_scale, sorted_ids, top_k, numel, post_pad, rows)
-            act = torch.empty((rows, inter), dtype=dtype, device=h.device)
-            _grouped_gemm(act, a1, w1, a1s, w1s, None, sorted_ids, expert_ids, post_pad, numel,
-                          scale_mode, fuse_silu=True, scatter=False, mul_weight=False)
-            if scale_mode == _cabi.SCALE_BLOCK:
-                a2, a2s = _group_quant(act, 128, None, 1, 0, post_pad, rows)
-            elif scale_mode == _cabi.SCALE_VECTOR:
-                a2, a2s = quant_rows(act, None, 1, 0, post_pad, rows)
-            else:
-                a2, a2s = _per_tensor_quant(act, a2_scale, None, 1, 0, post_pad, rows, amax_rows_dev=post_pad)
-            routed = torch.empty((t, top_k, k_out), dtype=dtype, device=h.device)
-            _grouped_gemm(routed, a2, w2, a2s, w2s, w, sorted_ids, expert_ids, post_pad, numel,
-                          scale_mode, fuse_silu=False, scatter=True, mul_weight=True)
-            moe_sum(routed, out[begin:end])
-    return out
+    return _run_experts(hidden_states, w1, w2, topk_weights, topk_ids, inplace, mode, w1s, w2s, scalar(a1_scale),
+                        scalar(a2_scale), global_num_experts, expert_map)
 
 
 def _dtype_of(compute_type):

@@ -247,8 +247,8 @@ int fg_ep_pack_rows_fp8_peer(const void* x, int x_dtype, int64_t T, int64_t K, i
 int64_t fg_moe_routed_workspace_bytes(int64_t n_rows_in, int num_experts, int64_t H, int64_t I);
 
 /* All experts local: y[T*topk, H] (route-slot order) = w2[e] . quant(silu_mul(w1[e] . quant(x)))
- * times the router weight, for every (token, slot).  Five launches (align, quantise+gather,
- * GEMM1+SiLU, quantise, GEMM2), no allocation: scratch is the caller's workspace (256-byte
+ * times the router weight, for every (token, slot).  Five launches (align, quantise, GEMM1+SiLU
+ * on gathered rows, quantise, GEMM2), no allocation: scratch is the caller's workspace (256-byte
  * aligned, fg_moe_routed_workspace_bytes(T*topk, ...)). */
 int fg_moe_routed_block_fp8_local(void* y, const void* hidden, int hidden_dtype, const void* topk_ids,
                                   int ids_are_i64, const void* topk_w, int topk_w_dtype, int64_t T,
@@ -256,19 +256,46 @@ int fg_moe_routed_block_fp8_local(void* y, const void* hidden, int hidden_dtype,
                                   const float* s2, int num_experts, int64_t H, int64_t I,
                                   void* workspace, int64_t workspace_bytes, void* stream);
 
+/* fused_experts_impl: src/flag_gems/fused/fused_moe.py:1821-2185, as one call in every weight format.
+ * out [T,H] (may be hidden itself) = sum over the topk slots of a token of router weight *
+ * w2[e] . q(silu_mul(w1[e] . q(hidden))), rows rounded to hidden_dtype before the fp32 sum (+ addend
+ * [T,H], nullable, joined in fp32).  w1 [local_experts, 2I, H], w2 [local_experts, H, I]; mode:
+ *   FG_EXPERTS_BLOCK_FP8    e4m3, scales [E, 2I/128, H/128] and [E, H/128, I/128], 1x128 activation groups
+ *   FG_EXPERTS_CHANNEL_FP8  e4m3, scales [E, 2I] and [E, H], one activation scale per token
+ *   FG_EXPERTS_CHANNEL_INT8 int8, the same layout
+ *   FG_EXPERTS_TENSOR_FP8   e4m3, scales [E]; activations by a1_scale / a2_scale[0], or dynamic when NULL
+ *   FG_EXPERTS_16BIT        bf16 / fp16 weights of hidden_dtype, no scales
+ *   FG_EXPERTS_16BIT_SCALED the same with scales [E, 2I] and [E, H] on the accumulators
+ * expert_map as in fg_moe_align_block_size (experts mapped to -1 contribute zeros).  Scratch is the
+ * caller's workspace (256-byte aligned, fg_fused_experts_workspace_bytes). */
+#define FG_EXPERTS_BLOCK_FP8 0
+#define FG_EXPERTS_CHANNEL_FP8 1
+#define FG_EXPERTS_CHANNEL_INT8 2
+#define FG_EXPERTS_TENSOR_FP8 3
+#define FG_EXPERTS_16BIT 4
+#define FG_EXPERTS_16BIT_SCALED 5
+int64_t fg_fused_experts_workspace_bytes(int mode, int64_t T, int topk, int num_experts, int64_t H,
+                                         int64_t I, int hidden_dtype);
+int fg_fused_experts(void* out, const void* hidden, int hidden_dtype, const void* topk_ids, int ids_are_i64,
+                     const void* topk_w, int topk_w_dtype, int64_t T, int topk, const void* w1,
+                     const void* w2, const float* s1, const float* s2, const float* a1_scale,
+                     const float* a2_scale, int mode, int num_experts, int local_experts,
+                     const int32_t* expert_map, int expert_map_len, int64_t H, int64_t I,
+                     const void* addend, void* workspace, int64_t workspace_bytes, void* stream);
+
 /* fg_moe_routed_block_fp8_local for callers that must not allocate device memory and have no
  * workspace to lend.  It has no counterpart in the reference.  Think of a host that handed the
  * whole device to its own memory planner at start-up (a later cudaMalloc fails or fragments its
  * plan), of code that runs where an allocation would stall every stream of the device, or of a
  * plug-in whose contract leaves all memory management to the embedding process.  The scratch is
  * a fixed array of FG_NOALLOC_SCRATCH_BYTES inside the library image (each GPU that loads the
- * library holds it until the process ends).  Problems whose scratch need (the value
+ * library holds it until the process ends).  Problems whose scratch need (at most the value
  * fg_moe_routed_workspace_bytes reports) exceeds it are refused with FG_ERR_UNSUPPORTED.
  * This function never calls cudaMalloc, cudaFree or any allocating routine.  Its first call on
  * a device looks up the array's device address (cudaGetSymbolAddress) and, like any first
  * launch, loads kernels: make that call before starting a stream capture.  All calls share the
- * one array and leave their intermediates in it; no part of it has to start at zero because a
- * call writes every element before reading it, but two calls whose kernels overlap on the GPU
+ * one array and leave their intermediates in it; no part of it has to start at zero because no
+ * element reaches a result before the call has written it, but two calls whose kernels overlap on the GPU
  * (different streams, or graphs replayed concurrently) race on it: keep them on one stream. */
 #define FG_NOALLOC_SCRATCH_BYTES (32u << 20)
 int fg_moe_routed_block_fp8_local_noalloc(void* y, const void* hidden, int hidden_dtype,
