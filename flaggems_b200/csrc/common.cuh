@@ -83,6 +83,12 @@ int fg_grouped_gemm(const FgGroupedGemm& g, cudaStream_t stream);
 int fg_group_tiles(const int32_t* offs, int num_groups, int64_t rows, int block, int32_t* sorted_ids, int64_t max_pad,
                    int32_t* expert_ids, int64_t n_blocks, int32_t* num_post_pad, cudaStream_t stream);
 
+// fg_moe_align_block_size_regions; fill_tail = false leaves the entries past the last block unwritten.
+int fg_moe_align(const void* topk_ids, int ids_are_i64, int64_t numel, int num_experts, int block_size, const int32_t* expert_map,
+                 int expert_map_len, int32_t* sorted_ids, int64_t max_pad, int32_t* expert_ids, int64_t n_blocks,
+                 int32_t* num_post_pad, int64_t ids_stride, int id_div, int32_t* expert_counts, const int32_t* numel_dev,
+                 int64_t region_rows, const int32_t* region_counts, int64_t region_stride, bool fill_tail, cudaStream_t stream);
+
 // x[0:n] = 1
 int fg_fill_ones(float* x, int64_t n, cudaStream_t stream);
 
@@ -100,6 +106,37 @@ int fg_quant_rows(int kind, const void* x, int x_dtype, void* q, float* s, const
 void fg_count_launch(int n);
 
 #ifdef __CUDACC__
+// Programmatic dependent launch: the kernels of this library are launched so that they may start while the
+// kernel before them in the stream is still running.  Each of them calls fg_pdl_wait() before it touches
+// global memory (it returns once every earlier kernel has finished and its writes are visible) and
+// fg_pdl_trigger() when the kernel after it may be scheduled.  What overlaps is launch latency and
+// prologues: ~2 us per kernel, which is a fifth of a decode-sized product.
+__device__ __forceinline__ void fg_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void fg_pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Launches `kernel` that way, with clusters of `cluster` CTAs when cluster > 1.
+template <typename... Params, typename... Args>
+cudaError_t fg_launch(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, unsigned cluster,
+                      Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.blockDim = dim3(block, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+    if (e == cudaSuccess) fg_count_launch(1);
+    return e;
+}
+
 template <typename T> struct FgVec8;  // eight elements of T as raw words
 
 __device__ __forceinline__ float fg_to_float(__nv_bfloat16 v) { return __bfloat162float(v); }

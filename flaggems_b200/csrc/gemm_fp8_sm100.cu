@@ -369,6 +369,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
     else __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_base_slot;
+    fg_pdl_wait();  // what precedes touches no global memory but the kernel's parameters
 
     const int num_k_blocks = (p.K + BLOCK_K - 1) / BLOCK_K;
     int num_m;
@@ -478,6 +479,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
             }
             FG_PROF_OUT(0, prof_wait);
         }
+        fg_pdl_trigger();  // every load of this CTA has been issued: only its last tile's epilogue is left
     } else if (ASTORE && warp == 3) {
         // ------------------------------- store warp -----------------------------------------
         // Writes parked tiles out: one 16-byte piece per lane, a whole row (or two) per instruction,
@@ -1229,20 +1231,7 @@ int launch_splitk(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams
             done = true;
         }
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(tiles * slices), 1, 1);
-    cfg.blockDim = dim3(C::THREADS, 1, 1);
-    cfg.dynamicSmemBytes = C::SMEM_BYTES;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)slices;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    FG_CUDA(cudaLaunchKernelEx(&cfg, kernel, ta, tb, p));
-    fg_count_launch(1);
+    FG_CUDA(fg_launch(kernel, (unsigned)(tiles * slices), C::THREADS, C::SMEM_BYTES, st, (unsigned)slices, ta, tb, p));
     return FG_OK;
 }
 
@@ -1260,7 +1249,6 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& 
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(C::THREADS, 1, 1);
     cfg.dynamicSmemBytes = C::SMEM_BYTES;
-    cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
@@ -1279,9 +1267,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& 
         max_clusters = n < fg_num_sms() / 2 ? n : fg_num_sms() / 2;
     }
     const int clusters = pair_tiles < max_clusters ? pair_tiles : max_clusters;
-    cfg.gridDim = dim3((unsigned)(2 * clusters), 1, 1);
-    FG_CUDA(cudaLaunchKernelEx(&cfg, kernel, ta, tb, p));
-    fg_count_launch(1);
+    FG_CUDA(fg_launch(kernel, (unsigned)(2 * clusters), C::THREADS, C::SMEM_BYTES, st, 2, ta, tb, p));
     return FG_OK;
 }
 
@@ -1312,9 +1298,7 @@ int launch_inst(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& 
     int grid = fg_num_sms();
     if (max_tiles < grid) grid = max_tiles;
     if (grid < 1) grid = 1;
-    kernel<<<grid, C::THREADS, C::SMEM_BYTES, st>>>(ta, tb, p);
-    fg_count_launch(1);
-    FG_LAUNCH_CHECK();
+    FG_CUDA(fg_launch(kernel, (unsigned)grid, C::THREADS, C::SMEM_BYTES, st, 1, ta, tb, p));
     return FG_OK;
 }
 

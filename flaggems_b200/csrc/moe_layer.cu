@@ -274,8 +274,8 @@ int fg_moe_routed_block_fp8_local(void* y, const void* hidden, int hidden_dtype,
     const Workspace ws = carve(workspace, n_in, num_experts, H, I, 2);
     FG_REQUIRE(workspace_bytes >= ws.bytes, FG_ERR_INVALID_ARGUMENT, "workspace holds %lld bytes, needs %lld",
                (long long)workspace_bytes, (long long)ws.bytes);
-    rc = fg_moe_align_block_size(topk_ids, ids_are_i64, n_in, num_experts, TILE_ROWS, nullptr, 0, ws.sorted_ids,
-                                 ws.max_pad, ws.expert_ids, ws.n_blocks, ws.post_pad, stream);
+    rc = fg_moe_align(topk_ids, ids_are_i64, n_in, num_experts, TILE_ROWS, nullptr, 0, ws.sorted_ids, ws.max_pad, ws.expert_ids,
+                      ws.n_blocks, ws.post_pad, 1, 1, nullptr, nullptr, 0, nullptr, 0, false, (cudaStream_t)stream);
     if (rc != FG_OK) return rc;
     const Experts e{FG_EXPERTS_BLOCK_FP8, hidden, hidden_dtype, topk_w, topk_w_dtype, T, topk, w1, w2, s1, s2, nullptr, nullptr,
                     num_experts, H, I, use_gather(n_in, num_experts)};
@@ -392,8 +392,9 @@ int fg_fused_experts(void* out, const void* hidden, int hidden_dtype, const void
     const Workspace ws = carve_experts(workspace, mode, T, topk, num_experts, H, I, hidden_dtype == FG_DTYPE_F32 ? 4 : 2);
     FG_REQUIRE((uintptr_t)workspace % 256 == 0 && workspace_bytes >= ws.bytes, FG_ERR_INVALID_ARGUMENT,
                "workspace holds %lld bytes, needs %lld (256-byte aligned)", (long long)workspace_bytes, (long long)ws.bytes);
-    int rc = fg_moe_align_block_size(topk_ids, ids_are_i64, T * topk, num_experts, TILE_ROWS, expert_map, expert_map_len,
-                                     ws.sorted_ids, ws.max_pad, ws.expert_ids, ws.n_blocks, ws.post_pad, stream);
+    int rc = fg_moe_align(topk_ids, ids_are_i64, T * topk, num_experts, TILE_ROWS, expert_map, expert_map_len, ws.sorted_ids,
+                          ws.max_pad, ws.expert_ids, ws.n_blocks, ws.post_pad, 1, 1, nullptr, nullptr, 0, nullptr, 0, false,
+                          (cudaStream_t)stream);
     if (rc != FG_OK) return rc;
     const Experts e{mode, hidden, hidden_dtype, topk_w, topk_w_dtype, T, topk, w1, w2, s1, s2, a1_scale, a2_scale,
                     local_experts, H, I, use_gather(T * topk, num_experts)};

@@ -136,6 +136,8 @@ __device__ __forceinline__ int64_t source_row(const QuantArgs& a, int64_t r) {
 // a constant stride and keeps (row, column group) incrementally: no division in the loop.
 template <typename T, int MODE, int TPG, int VPT>
 __global__ void __launch_bounds__(256) group_quant_kernel(QuantArgs a) {
+    fg_pdl_wait();
+    fg_pdl_trigger();
     constexpr int UNROLL = 2;
     constexpr int GROUP = TPG * 8 * VPT;
     const int64_t rows = resolve_rows(a);
@@ -218,6 +220,8 @@ __global__ void __launch_bounds__(256) group_quant_kernel(QuantArgs a) {
 // raw 16-bit pairs; a team of eight lanes owns a group.
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256, 5) group_pack16_kernel(QuantArgs a) {
+    fg_pdl_wait();
+    fg_pdl_trigger();
     constexpr int UNROLL = 2, TPG = 8;
     constexpr int GROUP = TPG * 16;
     using P = Pair16<T>;
@@ -300,6 +304,8 @@ __global__ void __launch_bounds__(256, 5) group_pack16_kernel(QuantArgs a) {
 // r (a local packed buffer, or this rank's region of the destination rank's receive buffer) and
 // writes the row's trailer.  One warp per row, four 16-byte loads in flight per lane.
 __global__ void __launch_bounds__(256) pack_copy_kernel(QuantArgs a, const uint8_t* __restrict__ staged) {
+    fg_pdl_wait();
+    fg_pdl_trigger();
     const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const int nvec = (int)(a.K / 16);
     const int s_cols = (int)(a.K / a.group);
@@ -333,6 +339,8 @@ __global__ void __launch_bounds__(256) pack_copy_kernel(QuantArgs a, const uint8
 // ---- any group size (multiple of 8), one CTA per group: per-token rows, block_size = K ...
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256) row_quant_kernel(QuantArgs a) {
+    fg_pdl_wait();
+    fg_pdl_trigger();
     constexpr int MAXV = 8;  // vectors of 8 cached in registers per thread
     const int64_t rows = resolve_rows(a);
     const int64_t gpr = a.K / a.group;
@@ -460,6 +468,8 @@ __device__ __forceinline__ typename Pair16<T>::V absmax16(typename Pair16<T>::V 
 // this runs at 6 (8192 x 4096).
 template <typename T, int MODE, int TPG>
 __global__ void __launch_bounds__(1024) group_row16_kernel(QuantArgs a) {
+    fg_pdl_wait();
+    fg_pdl_trigger();
     const int64_t row = blockIdx.x;
     if (row >= resolve_rows(a)) return;
     const int64_t src = source_row(a, row);
@@ -489,6 +499,8 @@ __global__ void __launch_bounds__(1024) group_row16_kernel(QuantArgs a) {
 
 template <typename T, int MODE>
 __global__ void __launch_bounds__(1024) row_quant16_kernel(QuantArgs a) {
+    fg_pdl_wait();
+    fg_pdl_trigger();
     using P = Pair16<T>;
     constexpr bool TENSOR = MODE == QM_TENSOR_STATIC || MODE == QM_TENSOR_DYNAMIC;
     const int64_t row = blockIdx.x;
@@ -549,21 +561,18 @@ int launch_rows(int dtype, const QuantArgs& a, cudaStream_t st) {
     const unsigned rows = (unsigned)a.rows;
     const int64_t threads = fg_cdiv(fg_cdiv(a.K, 16 * ROW_UNITS), 32) * 32;
     const bool wide = a.K % 16 == 0 && threads <= 1024 && (uintptr_t)a.q % 16 == 0 && a.ld_q % 16 == 0;
+    auto go = [&](auto kernel, unsigned block) -> int {
+        FG_CUDA(fg_launch(kernel, rows, block, 0, st, 1, a));
+        return FG_OK;
+    };
     switch (dtype) {
         case FG_DTYPE_BF16:
-            if (wide) row_quant16_kernel<__nv_bfloat16, MODE><<<rows, (unsigned)threads, 0, st>>>(a);
-            else row_quant_kernel<__nv_bfloat16, MODE><<<rows, 256, 0, st>>>(a);
-            break;
+            return wide ? go(row_quant16_kernel<__nv_bfloat16, MODE>, (unsigned)threads) : go(row_quant_kernel<__nv_bfloat16, MODE>, 256);
         case FG_DTYPE_F16:
-            if (wide) row_quant16_kernel<__half, MODE><<<rows, (unsigned)threads, 0, st>>>(a);
-            else row_quant_kernel<__half, MODE><<<rows, 256, 0, st>>>(a);
-            break;
-        case FG_DTYPE_F32: row_quant_kernel<float, MODE><<<rows, 256, 0, st>>>(a); break;
+            return wide ? go(row_quant16_kernel<__half, MODE>, (unsigned)threads) : go(row_quant_kernel<__half, MODE>, 256);
+        case FG_DTYPE_F32: return go(row_quant_kernel<float, MODE>, 256);
         default: fg_set_error("unsupported input dtype code %d", dtype); return FG_ERR_INVALID_ARGUMENT;
     }
-    fg_count_launch(1);
-    FG_LAUNCH_CHECK();
-    return FG_OK;
 }
 
 // Global max|x| over rows [0, rows) into amax[0] (which must start at zero): block reduction, then
@@ -572,6 +581,8 @@ template <typename T>
 __global__ void __launch_bounds__(256) abs_max_kernel(const T* __restrict__ x, int64_t rows, int64_t K, int64_t ld_x,
                                                       const int32_t* __restrict__ n_rows_dev,
                                                       unsigned int* __restrict__ amax) {
+    fg_pdl_wait();
+    fg_pdl_trigger();
     if (n_rows_dev) {
         const int64_t v = *n_rows_dev;
         rows = v < rows ? v : rows;
@@ -606,17 +617,13 @@ int launch_quant_t(const QuantArgs& a, cudaStream_t st) {
         const int64_t cap = (int64_t)fg_num_sms() * 24;
         if (blocks > cap) blocks = cap;
         if (blocks < 1) blocks = 1;
-        kernel<<<(unsigned)blocks, 256, 0, st>>>(a);
-        fg_count_launch(1);
-        FG_LAUNCH_CHECK();
+        FG_CUDA(fg_launch(kernel, (unsigned)blocks, 256, 0, st, 1, a));
         return FG_OK;
     };
     if constexpr (sizeof(T) == 2) {
         const int64_t threads = fg_cdiv(fg_cdiv(a.K, 16 * ROW_UNITS), 32) * 32;
         auto by_row = [&](auto kernel) -> int {
-            kernel<<<(unsigned)a.rows, (unsigned)threads, 0, st>>>(a);
-            fg_count_launch(1);
-            FG_LAUNCH_CHECK();
+            FG_CUDA(fg_launch(kernel, (unsigned)a.rows, (unsigned)threads, 0, st, 1, a));
             return FG_OK;
         };
         // 16-byte stores need 16-byte aligned output rows; otherwise the generic kernel below
@@ -643,9 +650,7 @@ int launch_quant_t(const QuantArgs& a, cudaStream_t st) {
         default: break;
     }
     FG_REQUIRE(groups < (1ll << 31), FG_ERR_UNSUPPORTED, "too many groups (%lld) for one launch", (long long)groups);
-    row_quant_kernel<T, MODE><<<(unsigned)groups, 256, 0, st>>>(a);
-    fg_count_launch(1);
-    FG_LAUNCH_CHECK();
+    FG_CUDA(fg_launch(row_quant_kernel<T, MODE>, (unsigned)groups, 256, 0, st, 1, a));
     return FG_OK;
 }
 
@@ -774,9 +779,7 @@ int fg_ep_pack_rows_fp8_peer(const void* x, int x_dtype, int64_t T, int64_t K, i
         int64_t blocks = fg_cdiv(a.rows, 8);
         const int64_t cap = (int64_t)fg_num_sms() * 8;
         if (blocks > cap) blocks = cap;
-        pack_copy_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(a, (const uint8_t*)packed);
-        fg_count_launch(1);
-        FG_LAUNCH_CHECK();
+        FG_CUDA(fg_launch(pack_copy_kernel, (unsigned)blocks, 256, 0, (cudaStream_t)stream, 1, a, (const uint8_t*)packed));
         return FG_OK;
     }
     return launch_quant<QM_GROUP>(x_dtype, a, (cudaStream_t)stream);
@@ -795,13 +798,11 @@ int fg_abs_max(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ld_x, c
     cudaStream_t st = (cudaStream_t)stream;
     unsigned int* out = reinterpret_cast<unsigned int*>(amax);
     switch (x_dtype) {
-        case FG_DTYPE_BF16: abs_max_kernel<<<(unsigned)blocks, 256, 0, st>>>((const __nv_bfloat16*)x, M, K, ld_x, n_rows_dev, out); break;
-        case FG_DTYPE_F16: abs_max_kernel<<<(unsigned)blocks, 256, 0, st>>>((const __half*)x, M, K, ld_x, n_rows_dev, out); break;
-        case FG_DTYPE_F32: abs_max_kernel<<<(unsigned)blocks, 256, 0, st>>>((const float*)x, M, K, ld_x, n_rows_dev, out); break;
+        case FG_DTYPE_BF16: FG_CUDA(fg_launch(abs_max_kernel<__nv_bfloat16>, (unsigned)blocks, 256, 0, st, 1, (const __nv_bfloat16*)x, M, K, ld_x, n_rows_dev, out)); break;
+        case FG_DTYPE_F16: FG_CUDA(fg_launch(abs_max_kernel<__half>, (unsigned)blocks, 256, 0, st, 1, (const __half*)x, M, K, ld_x, n_rows_dev, out)); break;
+        case FG_DTYPE_F32: FG_CUDA(fg_launch(abs_max_kernel<float>, (unsigned)blocks, 256, 0, st, 1, (const float*)x, M, K, ld_x, n_rows_dev, out)); break;
         default: fg_set_error("unsupported input dtype code %d", x_dtype); return FG_ERR_INVALID_ARGUMENT;
     }
-    fg_count_launch(1);
-    FG_LAUNCH_CHECK();
     return FG_OK;
 }
 
