@@ -102,6 +102,10 @@ int fg_quant_rows(int kind, const void* x, int x_dtype, void* q, float* s, const
                   int64_t K, const int32_t* row_index, int32_t index_div, int32_t index_limit, const int32_t* n_rows_dev,
                   cudaStream_t st);
 
+// fg_abs_max over the rows row_index names (entries outside [0, index_limit) are skipped); NULL: rows 0 .. M - 1.
+int fg_abs_max_rows(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ld_x, const int32_t* n_rows_dev,
+                    const int32_t* row_index, int32_t index_limit, float* amax, cudaStream_t st);
+
 // Adds n to the process-wide count of kernels launched by this library.
 void fg_count_launch(int n);
 

@@ -489,6 +489,7 @@ PyObject* fused_experts(PyObject*, PyObject* const* p, Py_ssize_t n) {
         const at::Tensor* map = nullptr;
         if (p[12] != Py_None && !(map = cuda_tensor(p[12]))) return none();
         const int64_t t = x->size(0), h = x->size(1), inter = w2->size(2), topk = ids->size(1);
+        if (experts < w1->size(0)) experts = w1->size(0);  // more weights than the count names: ids stay below it
         const int code = dtype_code(x->scalar_type()), esz = (int)x->element_size();
         const bool i64 = ids->scalar_type() == ScalarType::Long;
         c10::cuda::CUDAGuard guard(x->device());

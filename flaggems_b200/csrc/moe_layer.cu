@@ -104,10 +104,12 @@ struct Experts {
 // The line between the two row orders (see the head of this file).
 bool use_gather(int64_t slots, int num_experts) { return slots <= 32 * (int64_t)num_experts; }
 
-// Rows of one GEMM's input in the operand type of the mode; *scale is where their scales are.
+// Rows of one GEMM's input in the operand type of the mode; *scale is where their scales are.  `slots` (NULL or the
+// alignment table): only the rows that it names count toward a dynamic per-tensor scale.  In route-slot
+// order a slot whose expert id is out of range has a row that nothing wrote.
 int quantise(int mode, const void* x, int dtype, uint8_t* q, float* s, float* scalars, const float* given, int64_t src_rows,
              int64_t rows, int64_t K, const int32_t* index, int div, int64_t limit, const int32_t* n_rows_dev, const float** scale,
-             cudaStream_t st) {
+             cudaStream_t st, const Workspace* slots = nullptr) {
     *scale = s;
     const int kind = mode == FG_EXPERTS_BLOCK_FP8 ? FG_QUANT_GROUP128 : mode == FG_EXPERTS_CHANNEL_FP8 ? FG_QUANT_TOKEN
                      : mode == FG_EXPERTS_CHANNEL_INT8 ? FG_QUANT_INT8 : FG_QUANT_TENSOR;
@@ -116,7 +118,9 @@ int quantise(int mode, const void* x, int dtype, uint8_t* q, float* s, float* sc
         *scale = given ? given : scalars + 1;
         if (!given) {  // scalars[0]: amax, scalars[1]: the scale derived from it
             FG_CUDA(cudaMemsetAsync(scalars, 0, 4, st));
-            const int rc = fg_abs_max(x, dtype, src_rows, K, K, index && div == 0 ? n_rows_dev : nullptr, scalars, st);
+            const int rc = slots ? fg_abs_max_rows(x, dtype, slots->max_pad, K, K, slots->post_pad, slots->sorted_ids, (int32_t)src_rows,
+                                                   scalars, st)
+                                 : fg_abs_max(x, dtype, src_rows, K, K, index && div == 0 ? n_rows_dev : nullptr, scalars, st);
             if (rc != FG_OK) return rc;
             tensor = scalars;
         }
@@ -178,7 +182,7 @@ int run_experts(const Experts& e, const Workspace& ws, void* y, cudaStream_t st)
     if (rc != FG_OK) return rc;
     if (!plain) {
         if (e.gathered) rc = quantise(e.mode, ws.act, e.dtype, ws.a2, ws.a2s, ws.scalars + 2, e.a2_scale, slots, slots, e.I, nullptr, 1,
-                                      0, nullptr, &a2s, st);
+                                      0, nullptr, &a2s, st, &ws);
         else rc = quantise(e.mode, ws.act, e.dtype, ws.a2, ws.a2s, ws.scalars + 2, e.a2_scale, ws.rows, ws.rows, e.I, ws.sorted_ids, 0,
                            slots, ws.post_pad, &a2s, st);
         if (rc != FG_OK) return rc;

@@ -577,9 +577,11 @@ int launch_rows(int dtype, const QuantArgs& a, cudaStream_t st) {
 
 // Global max|x| over rows [0, rows) into amax[0] (which must start at zero): block reduction, then
 // one atomicMax per block on the bit pattern (non-negative floats order like unsigned integers).
+// With row_index: over the rows that it names, entries outside [0, index_limit) skipped.
 template <typename T>
 __global__ void __launch_bounds__(256) abs_max_kernel(const T* __restrict__ x, int64_t rows, int64_t K, int64_t ld_x,
                                                       const int32_t* __restrict__ n_rows_dev,
+                                                      const int32_t* __restrict__ row_index, int32_t index_limit,
                                                       unsigned int* __restrict__ amax) {
     fg_pdl_wait();
     fg_pdl_trigger();
@@ -591,7 +593,12 @@ __global__ void __launch_bounds__(256) abs_max_kernel(const T* __restrict__ x, i
     float m = 0.0f;
     for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < total; v += (int64_t)gridDim.x * blockDim.x) {
         float f[8];
-        fg_load8(x + (v / vec_per_row) * ld_x + (v % vec_per_row) * 8, f);
+        int64_t row = v / vec_per_row;
+        if (row_index) {
+            row = row_index[row];
+            if (row < 0 || row >= index_limit) continue;
+        }
+        fg_load8(x + row * ld_x + (v % vec_per_row) * 8, f);
 #pragma unroll
         for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(f[i]));
     }
@@ -787,6 +794,13 @@ int fg_ep_pack_rows_fp8_peer(const void* x, int x_dtype, int64_t T, int64_t K, i
 
 int fg_abs_max(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ld_x, const int32_t* n_rows_dev,
                float* amax, void* stream) {
+    return fg_abs_max_rows(x, x_dtype, M, K, ld_x, n_rows_dev, nullptr, 0, amax, (cudaStream_t)stream);
+}
+
+}  // extern "C"
+
+int fg_abs_max_rows(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ld_x, const int32_t* n_rows_dev,
+                    const int32_t* row_index, int32_t index_limit, float* amax, cudaStream_t st) {
     FG_REQUIRE(M >= 0 && K >= 0 && amax, FG_ERR_INVALID_ARGUMENT, "bad arguments");
     if (M == 0 || K == 0) return FG_OK;
     const int esz = x_dtype == FG_DTYPE_F32 ? 4 : 2;
@@ -795,16 +809,17 @@ int fg_abs_max(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ld_x, c
     int64_t blocks = fg_cdiv(M * (K / 8), 256 * 4);
     const int64_t cap = (int64_t)fg_num_sms() * 8;
     if (blocks > cap) blocks = cap;
-    cudaStream_t st = (cudaStream_t)stream;
     unsigned int* out = reinterpret_cast<unsigned int*>(amax);
     switch (x_dtype) {
-        case FG_DTYPE_BF16: FG_CUDA(fg_launch(abs_max_kernel<__nv_bfloat16>, (unsigned)blocks, 256, 0, st, 1, (const __nv_bfloat16*)x, M, K, ld_x, n_rows_dev, out)); break;
-        case FG_DTYPE_F16: FG_CUDA(fg_launch(abs_max_kernel<__half>, (unsigned)blocks, 256, 0, st, 1, (const __half*)x, M, K, ld_x, n_rows_dev, out)); break;
-        case FG_DTYPE_F32: FG_CUDA(fg_launch(abs_max_kernel<float>, (unsigned)blocks, 256, 0, st, 1, (const float*)x, M, K, ld_x, n_rows_dev, out)); break;
+        case FG_DTYPE_BF16: FG_CUDA(fg_launch(abs_max_kernel<__nv_bfloat16>, (unsigned)blocks, 256, 0, st, 1, (const __nv_bfloat16*)x, M, K, ld_x, n_rows_dev, row_index, index_limit, out)); break;
+        case FG_DTYPE_F16: FG_CUDA(fg_launch(abs_max_kernel<__half>, (unsigned)blocks, 256, 0, st, 1, (const __half*)x, M, K, ld_x, n_rows_dev, row_index, index_limit, out)); break;
+        case FG_DTYPE_F32: FG_CUDA(fg_launch(abs_max_kernel<float>, (unsigned)blocks, 256, 0, st, 1, (const float*)x, M, K, ld_x, n_rows_dev, row_index, index_limit, out)); break;
         default: fg_set_error("unsupported input dtype code %d", x_dtype); return FG_ERR_INVALID_ARGUMENT;
     }
     return FG_OK;
 }
+
+extern "C" {
 
 int fg_per_tensor_quant_fp8(const void* x, int x_dtype, void* q, const float* scale_or_amax, int dynamic,
                             float* scale_out, int64_t M, int64_t K, int64_t ld_x, int64_t ld_q,

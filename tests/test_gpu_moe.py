@@ -87,6 +87,26 @@ def test_fused_moe_per_tensor(static):
     _close(out, ref, rel=2e-2, strict_frac=0.99)
 
 
+def test_fused_moe_per_tensor_ignores_unrouted_slots():
+    # A slot with an expert id out of range has no row: what the workspace held there before must not
+    # reach the scale that all rows share.  More weights than `global_num_experts` are accepted too.
+    g = torch.Generator().manual_seed(4)
+    t, h, i, e, topk = 21, 256, 256, 8, 2
+    hidden = torch.randn(t, h, generator=g).bfloat16()
+    hidden[0] = 0
+    w1 = (torch.randn(e, 2 * i, h, generator=g) * 20).clamp(-448, 448).to(FP8).cuda()
+    w2 = (torch.randn(e, h, i, generator=g) * 20).clamp(-448, 448).to(FP8).cuda()
+    scales = dict(w1_scale=torch.full((e,), 1e-3, device="cuda"), w2_scale=torch.full((e,), 1e-3, device="cuda"))
+    tw, ti = _router(t, e - 1, topk, g)
+    ti[0] = -1
+    run = lambda a, b, c: flag_gems.fused_experts_impl(a.cuda(), w1, w2, b.cuda(), c.cuda(), use_fp8_w8a8=True,
+                                                       global_num_experts=e - 1, **scales)
+    ref = run(hidden[1:].contiguous(), tw[1:], ti[1:])
+    torch.full((64 << 20,), 3e38, dtype=torch.bfloat16, device="cuda")  # freed at once: the next workspace lies here
+    out = run(hidden, tw, ti)
+    assert torch.equal(out[1:], ref)
+
+
 @pytest.mark.parametrize("block_m", [16, 64, 128])
 @pytest.mark.parametrize("mode", ["block", "channel", "tensor"])
 def test_dispatch_fused_moe_kernel(block_m, mode):
