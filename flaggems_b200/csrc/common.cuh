@@ -69,6 +69,7 @@ struct FgGroupedGemm {
     int64_t N, K, ld_a, ld_as, ld_c;  // ld_as: block scales only
     int operand;  // 0 e4m3, 1 int8, 2 bf16, 3 fp16
     int block_rows, scale_mode, a_scale_per_row, fuse_silu, scatter, mul_weight, out_dtype;
+    int cta_pairs;  // block_rows = 256: every block is one tile row of a CTA pair
     const float* bias;  // fp32, added before the cast; bias_stride elements between the rows of consecutive experts
     int64_t bias_stride;
     const int32_t* dest;

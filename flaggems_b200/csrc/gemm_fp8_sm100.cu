@@ -82,7 +82,7 @@ struct GemmParams {
     const int32_t* sorted_ids;
     const int32_t* expert_ids;
     const int32_t* num_post_pad;
-    int block_rows;  // grouped: rows per m-tile (TMA box rows of A), <= 128
+    int block_rows;  // grouped: rows per m-tile (TMA box rows of A), <= 128; CTA pairs: 256, each CTA fetches its 128
     int a_box_rows;  // dense: TMA box rows of A (128, or fewer when M is small)
     int64_t numel;
     // Grouped, gather_div > 0: A (and its per-row scales) holds one row per token and route slot s reads
@@ -305,14 +305,14 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
     using C = Cfg<BN, SMALL_A, PAIR, ASTORE, !BLOCK_SCALED && !SPLITK>;
     static_assert(!ASTORE || (BLOCK_SCALED && !SPLITK), "the store warp serves the block-scaled tiles");
     constexpr bool INT8 = OPK == 1;
-    static_assert(OPK == 0 || (!BLOCK_SCALED && !SPLITK && !PAIR && !SMALL_A), "int8 and 16-bit operands serve the plain and grouped tiles");
+    static_assert(OPK == 0 || (!BLOCK_SCALED && !SPLITK && !SMALL_A), "int8 and 16-bit operands serve the plain and grouped tiles");
     // accumulator word -> fp32
     auto acc_f = [](uint32_t raw) -> float {
         if constexpr (INT8) return __int2float_rn((int)raw);
         else return __uint_as_float(raw);
     };
     static_assert(!SPLITK || (!FUSE_SILU && !SMALL_A && BN >= 128), "split-K is built for the plain wide tiles");
-    static_assert(!PAIR || (!SPLITK && !FUSE_SILU && !SMALL_A), "the CTA pair serves the plain dense tiles");
+    static_assert(!PAIR || (!SPLITK && !BLOCK_SCALED && !SMALL_A), "the CTA pair serves the tiles without block scales");
     static_assert(!FUSE_SILU || BN >= 128, "fused SiLU needs a tile of at least 128 columns");
     constexpr int STAGES = C::STAGES;
     constexpr int OUT_TILE_N = FUSE_SILU ? BN / 2 : BN;  // output columns per tile
@@ -380,7 +380,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
     } else {
         num_m = (int)((p.M + BLOCK_M - 1) / BLOCK_M);
     }
-    if constexpr (PAIR) num_m = (int)((p.M + 2 * BLOCK_M - 1) / (2 * BLOCK_M));
+    if (PAIR && !p.grouped) num_m = (int)((p.M + 2 * BLOCK_M - 1) / (2 * BLOCK_M));
     const int num_n = (p.n_out + OUT_TILE_N - 1) / OUT_TILE_N;
     const int num_tiles = num_m * num_n;
     const int a_rows_step = PAIR ? 2 * BLOCK_M : (p.grouped ? p.block_rows : BLOCK_M);
@@ -399,7 +399,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
         tile_first = blockIdx.x / k_slices;
         tile_step = gridDim.x / k_slices;
     }
-    const uint32_t stage_tx = (uint32_t)((p.grouped ? p.block_rows : p.a_box_rows) * BLOCK_K + C::B_BYTES);
+    const uint32_t stage_tx = (uint32_t)((PAIR ? BLOCK_M : p.grouped ? p.block_rows : p.a_box_rows) * BLOCK_K + C::B_BYTES);
 
     if (warp < C::FIRST_EPI_WARP) {
       if constexpr (C::REBALANCE_REGS) setmaxnreg_dec<C::REGS_PRODUCER>();
@@ -449,7 +449,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                         const uint32_t bar0 = mapa_shared(smem_u32(&full_bar[stage]), 0u);
                         if (cta_rank == 0) mbar_arrive_expect_tx(&full_bar[stage], 2u * stage_tx);
                         tma_load_2d_2cta(sa, &tm_a, bar0, kb * BLOCK_K, m0);
-                        tma_load_3d_2cta(sb, &tm_b, bar0, kb * BLOCK_K, n0 + (int)cta_rank * (BN / 2), 0);
+                        // this CTA's 128 of the 256 rows of B; fused SiLU: gate rows here, up rows in the odd CTA
+                        tma_load_3d_2cta(sb, &tm_b, bar0, kb * BLOCK_K, n0 + (int)cta_rank * (FUSE_SILU ? p.N / 2 : BN / 2), expert);
                         if (++stage == STAGES) {
                             stage = 0;
                             phase ^= 1u;
@@ -595,9 +596,10 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
         // path: the state of the next K block's barriers is therefore probed (non-blocking)
         // before the current block's MMAs are issued, and the blocking wait is only the fallback.
         if (cta_rank == 0) {
-            constexpr uint32_t idesc = OPK == 1 ? umma_idesc_s8_s32(BLOCK_M, BN)
-                                       : OPK >= 2 ? umma_idesc_16bit_f32(BLOCK_M, BN, OPK == 2)
-                                                  : umma_idesc_e4m3_f32(PAIR ? 2 * BLOCK_M : BLOCK_M, BN);
+            constexpr int MMA_M = PAIR ? 2 * BLOCK_M : BLOCK_M;
+            constexpr uint32_t idesc = OPK == 1 ? umma_idesc_s8_s32(MMA_M, BN)
+                                       : OPK >= 2 ? umma_idesc_16bit_f32(MMA_M, BN, OPK == 2)
+                                                  : umma_idesc_e4m3_f32(MMA_M, BN);
             int stage = 0;
             uint32_t phase = 0;
             uint32_t acc_iter = 0;
@@ -614,7 +616,11 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                 for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
                     // advancing K by 32 bytes inside the swizzle row: +2 in 16-byte units
                     const uint32_t accumulate = (decltype(zero_first)::value && k == 0) ? 0u : 1u;
-                    if constexpr (PAIR)
+                    if constexpr (PAIR && INT8)
+                        umma_i8_2cta(d_tmem, a_desc + (uint64_t)(2 * k), b_desc + (uint64_t)(2 * k), idesc, accumulate);
+                    else if constexpr (PAIR && OPK >= 2)
+                        umma_f16_2cta(d_tmem, a_desc + (uint64_t)(2 * k), b_desc + (uint64_t)(2 * k), idesc, accumulate);
+                    else if constexpr (PAIR)
                         umma_f8f6f4_2cta(d_tmem, a_desc + (uint64_t)(2 * k), b_desc + (uint64_t)(2 * k), idesc, accumulate);
                     else if constexpr (INT8)
                         umma_i8(d_tmem, a_desc + (uint64_t)(2 * k), b_desc + (uint64_t)(2 * k), idesc, accumulate);
@@ -1236,12 +1242,13 @@ int launch_splitk(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams
 }
 
 // CTA-pair kernel: clusters of two, one cluster per 256 x 256 tile, persistent over the tiles.
-// Dense scales only: with block scales the accumulator of every K block has to make the round
+// No block scales: with block scales the accumulator of every K block has to make the round
 // trip MMA -> both CTAs' epilogues -> MMA through cluster-wide barriers, and that latency costs
 // more than the halved B traffic saves (measured: about half the single-CTA throughput).
+template <bool SILU, int OPK>
 int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int pair_tiles, cudaStream_t st) {
     using C = Cfg<256, false, true, false, true>;
-    auto kernel = gemm_fp8_kernel<256, false, false, false, false, true>;
+    auto kernel = gemm_fp8_kernel<256, false, SILU, false, false, true, false, OPK>;
     static int max_clusters_dev[64];
     static std::mutex mu;
     std::lock_guard<std::mutex> lock(mu);
@@ -1320,7 +1327,11 @@ int launch_gemm(GemmParams& p, const void* a, int64_t a_rows, int64_t ld_a, cons
     const int64_t enough = (int64_t)sms * 5 / 8;
     int bn;
     bool small_a = false;
-    if (fuse_silu) {
+    const bool grouped_pair = p.grouped && p.block_rows == 2 * BLOCK_M;  // the caller aligned its rows to 256 per expert
+    FG_REQUIRE(!grouped_pair || (!block_scaled && (p.gather_div == 0 || p.a_contiguous)), FG_ERR_UNSUPPORTED, "256-row blocks are for CTA pairs");
+    if (grouped_pair) {
+        bn = 256;
+    } else if (fuse_silu) {
         bn = m_tiles * fg_cdiv(p.n_out, 128) >= enough ? 256 : 128;
     } else if (m_tiles * fg_cdiv(p.n_out, 256) >= enough) {
         bn = 256;
@@ -1357,9 +1368,9 @@ int launch_gemm(GemmParams& p, const void* a, int64_t a_rows, int64_t ld_a, cons
     // Large dense products: a pair of CTAs per 256 x 256 tile (a third less L2 and shared-memory
     // traffic per flop: +4-5 % under the power cap) once there are at least three waves of such
     // tiles; with fewer, the coarser tiles lose more to the ragged last wave than they gain.
-    const int64_t pair_tiles = fg_cdiv(p.M, 2 * BLOCK_M) * fg_cdiv(p.n_out, 256);
-    const bool pair = !p.grouped && !fuse_silu && !block_scaled && bn == 256 && k_slices == 1 &&
-                      pair_tiles >= 3 * (int64_t)(sms / 2) && pair_tiles < (1ll << 30) && pair_enabled();
+    const int64_t pair_tiles = fg_cdiv(p.M, 2 * BLOCK_M) * fg_cdiv(p.n_out, fuse_silu ? 128 : 256);
+    const bool pair = grouped_pair || (!p.grouped && !fuse_silu && !block_scaled && bn == 256 && k_slices == 1 &&
+                                       pair_tiles >= 3 * (int64_t)(sms / 2) && pair_tiles < (1ll << 30) && pair_enabled());
     const int out_tile = fuse_silu ? bn / 2 : bn;
     const int64_t tiles = m_tiles * fg_cdiv(p.n_out, out_tile);
     FG_REQUIRE(tiles < (1ll << 31), FG_ERR_UNSUPPORTED, "too many tiles");
@@ -1367,12 +1378,24 @@ int launch_gemm(GemmParams& p, const void* a, int64_t a_rows, int64_t ld_a, cons
 
     CUtensorMap ta, tb;
     int rc = make_map(&ta, a, (uint64_t)p.K, (uint64_t)a_rows, 1, (uint64_t)ld_a, 0,
-                      (uint32_t)(p.gather_div > 0 && !p.a_contiguous ? 1 : p.grouped ? p.block_rows : p.a_box_rows), 2);
+                      (uint32_t)(p.gather_div > 0 && !p.a_contiguous ? 1 : pair ? BLOCK_M : p.grouped ? p.block_rows : p.a_box_rows), 2);
     if (rc != FG_OK) return rc;
     rc = make_map(&tb, b, (uint64_t)p.K, (uint64_t)p.N, (uint64_t)num_experts, (uint64_t)ld_b,
                   (uint64_t)ld_b * (uint64_t)p.N, (uint32_t)((fuse_silu || pair) ? bn / 2 : bn), 3);
     if (rc != FG_OK) return rc;
-    if (pair) return launch_pair(ta, tb, p, (int)pair_tiles, st);
+    if (pair) {
+        FG_REQUIRE(pair_tiles < (1ll << 30), FG_ERR_UNSUPPORTED, "too many tiles");
+        auto by_kind = [&](auto silu_tag) -> int {
+            constexpr bool S = decltype(silu_tag)::value;
+            switch (p.int8) {
+                case 0: return launch_pair<S, 0>(ta, tb, p, (int)pair_tiles, st);
+                case 1: return launch_pair<S, 1>(ta, tb, p, (int)pair_tiles, st);
+                case 2: return launch_pair<S, 2>(ta, tb, p, (int)pair_tiles, st);
+                default: return launch_pair<S, 3>(ta, tb, p, (int)pair_tiles, st);
+            }
+        };
+        return fuse_silu ? by_kind(std::true_type()) : by_kind(std::false_type());
+    }
 
     const int t = (int)tiles;
     if (p.int8) {
@@ -1545,8 +1568,8 @@ int fg_grouped_gemm(const FgGroupedGemm& g, cudaStream_t stream) {
                FG_ERR_INVALID_ARGUMENT,
                "peer scatter needs 1..8 peers, scatter mode, a (slot, rank) table and the peers' row capacity");
     FG_REQUIRE(dtype_ok(g.out_dtype), FG_ERR_INVALID_ARGUMENT, "bad out_dtype %d", g.out_dtype);
-    FG_REQUIRE(g.block_rows >= 8 && g.block_rows <= 128 && g.block_rows % 8 == 0, FG_ERR_UNSUPPORTED,
-               "block_rows %d must be a multiple of 8 in [8, 128]", g.block_rows);
+    FG_REQUIRE((g.block_rows >= 8 && g.block_rows <= 128 && g.block_rows % 8 == 0) || (g.block_rows == 2 * BLOCK_M && g.cta_pairs),
+               FG_ERR_UNSUPPORTED, "block_rows %d must be a multiple of 8 in [8, 128]", g.block_rows);
     FG_REQUIRE(!g.mul_weight || (g.topk_w && dtype_ok(g.topk_w_dtype)), FG_ERR_INVALID_ARGUMENT,
                "mul_weight needs topk_weights");
     FG_REQUIRE(g.N < (1ll << 31) && g.K < (1ll << 31), FG_ERR_UNSUPPORTED, "dimension too large");
@@ -1555,7 +1578,7 @@ int fg_grouped_gemm(const FgGroupedGemm& g, cudaStream_t stream) {
     FG_REQUIRE(!(block && g.fuse_silu) || (g.N / 2) % 128 == 0, FG_ERR_UNSUPPORTED,
                "fused SiLU with block scales needs the intermediate size %lld to be a multiple of 128",
                (long long)(g.N / 2));
-    FG_REQUIRE(g.gather_div == 0 || (g.gather_div > 0 && g.block_rows == BLOCK_M && (uintptr_t)g.sorted_ids % 16 == 0),
+    FG_REQUIRE(g.gather_div == 0 || (g.gather_div > 0 && (g.block_rows == BLOCK_M || g.cta_pairs) && (uintptr_t)g.sorted_ids % 16 == 0),
                FG_ERR_INVALID_ARGUMENT, "gathered rows need 128-row blocks and 16-byte aligned sorted_ids");
     if (g.max_rows == 0) return FG_OK;
     int64_t K = g.K, ld_a = g.ld_a;

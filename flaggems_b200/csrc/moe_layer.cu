@@ -23,6 +23,8 @@ static __device__ __align__(256) unsigned char g_routed_scratch[FG_NOALLOC_SCRAT
 namespace {
 
 constexpr int TILE_ROWS = 128;
+constexpr int PAIR_ROWS = 256;      // rows of a CTA pair's tile
+constexpr int PAIR_MIN_ROWS = 768;  // rows per expert from which pairs are used (see use_pairs)
 
 inline int64_t align_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
 
@@ -52,11 +54,11 @@ struct Carver {
 };
 
 // Sorted rows of `slots` route slots: every expert padded to the tile, and no more than one tile per slot.
-void carve_tables(Carver& c, Workspace& w, int64_t slots, int num_experts) {
-    w.max_pad = slots + (int64_t)num_experts * (TILE_ROWS - 1);
-    if (slots * TILE_ROWS < w.max_pad) w.max_pad = slots * TILE_ROWS;
-    w.n_blocks = fg_cdiv(w.max_pad, TILE_ROWS);
-    w.rows = w.max_pad / TILE_ROWS * TILE_ROWS;
+void carve_tables(Carver& c, Workspace& w, int64_t slots, int num_experts, int tile = TILE_ROWS) {
+    w.max_pad = slots + (int64_t)num_experts * (tile - 1);
+    if (slots * tile < w.max_pad) w.max_pad = slots * tile;
+    w.n_blocks = fg_cdiv(w.max_pad, tile);
+    w.rows = w.max_pad / tile * tile;
     w.sorted_ids = (int32_t*)c.take(4 * w.max_pad);
     w.expert_ids = (int32_t*)c.take(4 * w.n_blocks);
     w.post_pad = (int32_t*)c.take(256);
@@ -98,8 +100,19 @@ struct Experts {
     const float *s1, *s2, *a1_scale, *a2_scale;
     int local_experts;
     int64_t H, I;
-    bool gathered;
+    bool gathered, pairs;
 };
+
+// Whether rows in expert order are padded to 256 per expert instead of 128 and the products run by CTA pairs:
+// `slots` rows against outputs of n1 and n2 columns.  A pair moves a third fewer operand bytes per flop and
+// pays 64 more padding rows per expert on average.  Steady state under the power cap, single -> pair: Mixtral,
+// 1024 rows per expert: fp8 1620 -> 1518 us, int8 1532 -> 1390, bf16 2875 -> 2710; 1024 rows per group x 4096 x 7168:
+// 256 -> 242; but 525 rows per expert: 984 -> 990, 500 rows per group x 4096 x 4096: 84.5 -> 89.  Hence 768
+// rows per expert, and three waves of pair tiles in the smaller product.
+bool use_pairs(int64_t slots, int num_experts, int64_t n1, int64_t n2) {
+    const int64_t n = n1 < n2 ? n1 : n2;
+    return slots >= PAIR_MIN_ROWS * (int64_t)num_experts && slots / PAIR_ROWS * (n / 256) >= 3 * (int64_t)(fg_num_sms() / 2);
+}
 
 // The line between the two row orders (see the head of this file).
 bool use_gather(int64_t slots, int num_experts) { return slots <= 32 * (int64_t)num_experts; }
@@ -173,7 +186,8 @@ int run_experts(const Experts& e, const Workspace& ws, void* y, cudaStream_t st)
 
     FgGroupedGemm g{};
     g.sorted_ids = ws.sorted_ids; g.expert_ids = ws.expert_ids; g.num_post_pad = ws.post_pad; g.max_rows = ws.rows;
-    g.numel = slots; g.num_experts = e.local_experts; g.block_rows = TILE_ROWS; g.out_dtype = e.dtype;
+    g.numel = slots; g.num_experts = e.local_experts; g.block_rows = e.pairs ? PAIR_ROWS : TILE_ROWS; g.cta_pairs = e.pairs;
+    g.out_dtype = e.dtype;
     g.operand = plain ? (e.dtype == FG_DTYPE_BF16 ? 2 : 3) : e.mode == FG_EXPERTS_CHANNEL_INT8 ? 1 : 0;
     g.scale_mode = block ? FG_SCALE_BLOCK : (unit || tensor) ? FG_SCALE_SCALAR : FG_SCALE_VECTOR;
     g.c = ws.act; g.a = a1; g.w = e.w1; g.a_scale = a1s; g.w_scale = s1; g.a_rows = e.T; g.gather_div = e.gathered ? e.topk : 0;
@@ -215,10 +229,10 @@ int builtin_scratch(void** out) {
 namespace {
 
 // Scratch of fg_scaled_grouped_mm_fp8: the alignment tables only.
-Workspace carve_grouped_mm(void* base, int64_t m_total, int num_groups) {
+Workspace carve_grouped_mm(void* base, int64_t m_total, int num_groups, int tile) {
     Workspace w{};
     Carver c{reinterpret_cast<uint8_t*>(base), 0};
-    carve_tables(c, w, m_total, num_groups);
+    carve_tables(c, w, m_total, num_groups, tile);
     w.bytes = c.off;
     return w;
 }
@@ -229,7 +243,8 @@ extern "C" {
 
 int64_t fg_scaled_grouped_mm_workspace_bytes(int64_t m_total, int num_groups, int64_t K) {
     if (m_total < 0 || num_groups <= 0 || K <= 0) return -1;
-    return carve_grouped_mm(nullptr, m_total, num_groups).bytes;
+    // the larger of the tables that the call may choose: its N is not known here
+    return carve_grouped_mm(nullptr, m_total, num_groups, m_total >= PAIR_MIN_ROWS * (int64_t)num_groups ? PAIR_ROWS : TILE_ROWS).bytes;
 }
 
 int fg_scaled_grouped_mm_fp8(void* c, const void* a, const void* b, const float* scale_a, const float* scale_b,
@@ -243,16 +258,18 @@ int fg_scaled_grouped_mm_fp8(void* c, const void* a, const void* b, const float*
     FG_REQUIRE(c && a && b && scale_a && scale_b && offs && workspace, FG_ERR_INVALID_ARGUMENT, "null pointer");
     FG_REQUIRE((uintptr_t)workspace % 256 == 0, FG_ERR_INVALID_ARGUMENT, "workspace must be 256-byte aligned");
     FG_REQUIRE(ld_a % 16 == 0 && (uintptr_t)a % 16 == 0, FG_ERR_UNSUPPORTED, "a must have 16-byte aligned rows");
-    const Workspace ws = carve_grouped_mm(workspace, m_total, num_groups);
+    const bool pairs = use_pairs(m_total, num_groups, N, N);
+    const int tile = pairs ? PAIR_ROWS : TILE_ROWS;
+    const Workspace ws = carve_grouped_mm(workspace, m_total, num_groups, tile);
     FG_REQUIRE(workspace_bytes >= ws.bytes, FG_ERR_INVALID_ARGUMENT, "workspace holds %lld bytes, needs %lld",
                (long long)workspace_bytes, (long long)ws.bytes);
     cudaStream_t st = (cudaStream_t)stream;
-    int rc = fg_group_tiles(offs, num_groups, m_total, TILE_ROWS, ws.sorted_ids, ws.max_pad, ws.expert_ids, ws.n_blocks,
+    int rc = fg_group_tiles(offs, num_groups, m_total, tile, ws.sorted_ids, ws.max_pad, ws.expert_ids, ws.n_blocks,
                             ws.post_pad, st);
     if (rc != FG_OK) return rc;
     FgGroupedGemm g{};
     g.sorted_ids = ws.sorted_ids; g.expert_ids = ws.expert_ids; g.num_post_pad = ws.post_pad; g.max_rows = ws.rows;
-    g.numel = m_total; g.num_experts = num_groups; g.block_rows = TILE_ROWS; g.scale_mode = FG_SCALE_VECTOR; g.out_dtype = out_dtype;
+    g.numel = m_total; g.num_experts = num_groups; g.block_rows = tile; g.cta_pairs = pairs; g.scale_mode = FG_SCALE_VECTOR; g.out_dtype = out_dtype;
     g.c = c; g.a = a; g.w = b; g.a_scale = scale_a; g.w_scale = scale_b; g.bias = bias; g.bias_stride = bias_stride_g;
     // few rows per group: only they are fetched; otherwise a block is one box from its first row
     g.a_rows = m_total; g.gather_div = 1; g.a_contiguous = !use_gather(m_total, num_groups); g.N = N; g.K = K; g.ld_a = ld_a; g.ld_c = ld_c; g.scatter = 1;
@@ -282,7 +299,7 @@ int fg_moe_routed_block_fp8_local(void* y, const void* hidden, int hidden_dtype,
                       ws.n_blocks, ws.post_pad, 1, 1, nullptr, nullptr, 0, nullptr, 0, false, (cudaStream_t)stream);
     if (rc != FG_OK) return rc;
     const Experts e{FG_EXPERTS_BLOCK_FP8, hidden, hidden_dtype, topk_w, topk_w_dtype, T, topk, w1, w2, s1, s2, nullptr, nullptr,
-                    num_experts, H, I, use_gather(n_in, num_experts)};
+                    num_experts, H, I, use_gather(n_in, num_experts), false};
     return run_experts(e, ws, y, (cudaStream_t)stream);
 }
 
@@ -360,9 +377,10 @@ static Workspace carve_experts(void* base, int mode, int64_t T, int topk, int nu
     Workspace w{};
     Carver c{reinterpret_cast<uint8_t*>(base), 0};
     const int64_t slots = T * topk;
+    const bool pairs = mode != FG_EXPERTS_BLOCK_FP8 && use_pairs(slots, num_experts, 2 * I, H);
     const bool gathered = use_gather(slots, num_experts), plain = mode == FG_EXPERTS_16BIT || mode == FG_EXPERTS_16BIT_SCALED;
     const int64_t cols1 = mode == FG_EXPERTS_BLOCK_FP8 ? H / 128 : 1, cols2 = mode == FG_EXPERTS_BLOCK_FP8 ? I / 128 : 1;
-    carve_tables(c, w, slots, num_experts);
+    carve_tables(c, w, slots, num_experts, pairs ? PAIR_ROWS : TILE_ROWS);
     const int64_t rows1 = gathered ? T : w.rows, rows2 = gathered ? slots : w.rows;
     w.scalars = (float*)c.take(4 * (num_experts > 64 ? num_experts : 64));
     w.a1 = c.take(plain ? (gathered ? 0 : rows1 * H * 2) : rows1 * H);
@@ -396,12 +414,13 @@ int fg_fused_experts(void* out, const void* hidden, int hidden_dtype, const void
     const Workspace ws = carve_experts(workspace, mode, T, topk, num_experts, H, I, hidden_dtype == FG_DTYPE_F32 ? 4 : 2);
     FG_REQUIRE((uintptr_t)workspace % 256 == 0 && workspace_bytes >= ws.bytes, FG_ERR_INVALID_ARGUMENT,
                "workspace holds %lld bytes, needs %lld (256-byte aligned)", (long long)workspace_bytes, (long long)ws.bytes);
-    int rc = fg_moe_align(topk_ids, ids_are_i64, T * topk, num_experts, TILE_ROWS, expert_map, expert_map_len, ws.sorted_ids,
+    const bool pairs = mode != FG_EXPERTS_BLOCK_FP8 && use_pairs(T * topk, num_experts, 2 * I, H);
+    int rc = fg_moe_align(topk_ids, ids_are_i64, T * topk, num_experts, pairs ? PAIR_ROWS : TILE_ROWS, expert_map, expert_map_len, ws.sorted_ids,
                           ws.max_pad, ws.expert_ids, ws.n_blocks, ws.post_pad, 1, 1, nullptr, nullptr, 0, nullptr, 0, false,
                           (cudaStream_t)stream);
     if (rc != FG_OK) return rc;
     const Experts e{mode, hidden, hidden_dtype, topk_w, topk_w_dtype, T, topk, w1, w2, s1, s2, a1_scale, a2_scale,
-                    local_experts, H, I, use_gather(T * topk, num_experts)};
+                    local_experts, H, I, use_gather(T * topk, num_experts), pairs};
     rc = run_experts(e, ws, ws.routed, (cudaStream_t)stream);
     if (rc != FG_OK) return rc;
     return fg_moe_sum_indexed(ws.routed, out, T, topk, H, hidden_dtype, nullptr, addend, stream);

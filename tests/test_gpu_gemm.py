@@ -382,3 +382,21 @@ def test_fp8_einsum_bhr_hdr_bhd():
         _close(z[:, i], oracle.block_scaled_mm(xq[:, i].contiguous(), yq[i], xs[:, i].contiguous(), ys[i]))
     with pytest.raises(AssertionError):
         flag_gems.fp8_einsum("bhr,hrd->bhd", xq.cuda(), xs.cuda(), yq.cuda(), ys.cuda())
+
+
+@pytest.mark.parametrize("offs", [[0, 129, 2400], [2048, 2049, 2049], [700, 1400, 2000]])
+def test_scaled_grouped_mm_cta_pairs(offs):
+    # 256-row blocks (2400 rows, three groups, N = 7168): empty and one-row groups, an empty second half, rows past the last end
+    g = torch.Generator(device="cuda").manual_seed(9)
+    m, n, k = 2400, 7168, 272
+    a = torch.randn(m, k, device="cuda", generator=g).to(torch.float8_e4m3fn)
+    b = torch.randn(3, n, k, device="cuda", generator=g).to(torch.float8_e4m3fn)
+    sa, sb = torch.rand(m, device="cuda", generator=g), torch.rand(3, n, device="cuda", generator=g)
+    out = flag_gems.scaled_grouped_mm(a, b.transpose(1, 2), sa, sb, torch.tensor(offs, dtype=torch.int32, device="cuda"))
+    lo = 0
+    for x, hi in enumerate(offs):
+        if hi > lo:
+            ref = (a[lo:hi].double() @ b[x].double().t()) * sa[lo:hi, None].double() * sb[x].double()
+            # fp32 sums of k products and one rounding to bf16
+            torch.testing.assert_close(out[lo:hi].double(), ref, rtol=2 ** -8, atol=1e-5 * k)
+        lo = hi

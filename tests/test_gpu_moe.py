@@ -394,3 +394,43 @@ def test_fused_moe_16bit_expert_map_inplace_and_empty():
     empty = flag_gems.fused_experts_impl(hidden[:0].cuda(), w1.cuda(), w2.cuda(), tw[:0].cuda(), ti[:0].cuda())
     assert empty.shape == (0, h)
     assert _cabi.device_status() == 0
+
+
+def _wide_experts(mode, e, h, i, g):
+    """Random experts of a mode on the GPU and the arguments that name it."""
+    def make(*shape):
+        if mode in ("bf16", "fp16"):
+            return (torch.randn(*shape, device="cuda", generator=g) * 0.02).to(torch.bfloat16 if mode == "bf16" else torch.float16)
+        if mode == "int8":
+            return torch.randint(-127, 128, shape, dtype=torch.int8, device="cuda", generator=g)
+        return torch.randn(*shape, device="cuda", generator=g).to(FP8)
+
+    w1, w2 = make(e, 2 * i, h), make(e, h, i)
+    if mode in ("bf16", "fp16"):
+        return w1, w2, {}
+    rand = lambda *s: torch.rand(*s, device="cuda", generator=g) * 1e-3 + 1e-3
+    if mode == "tensor":
+        return w1, w2, dict(use_fp8_w8a8=True, w1_scale=rand(e), w2_scale=rand(e), a1_scale=torch.full((1,), 0.01, device="cuda"),
+                            a2_scale=torch.full((1,), 0.05, device="cuda"))
+    kind = "use_int8_w8a8" if mode == "int8" else "use_fp8_w8a8"
+    return w1, w2, {kind: True, "per_channel_quant": True, "w1_scale": rand(e, 2 * i), "w2_scale": rand(e, h)}
+
+
+@pytest.mark.parametrize("mode", ["channel", "tensor", "int8", "bf16", "fp16"])
+def test_fused_moe_cta_pairs_match_single_ctas(mode):
+    # 3098 slots over 4 experts: blocks of 256 rows, some with an empty second half, I not a multiple of 128.
+    # Rows are independent, so 100 tokens at a time (128-row blocks) give the same bits.
+    g = torch.Generator(device="cuda").manual_seed(8)
+    t, e, h, i = 1549, 4, 7168, 3600
+    dtype = torch.float16 if mode == "fp16" else torch.bfloat16
+    x = torch.randn(t, h, device="cuda", generator=g).to(dtype)
+    w1, w2, how = _wide_experts(mode, e, h, i, g)
+    tw = torch.rand(t, 2, device="cuda", generator=g)
+    ti = torch.zeros(t, 2, dtype=torch.int64, device="cuda")  # rows per expert: 1549, 725, 724, 100
+    ti[:, 1] = 1 + torch.arange(t, device="cuda") % 2
+    ti[:100, 1] = 3
+    out = flag_gems.fused_experts_impl(x, w1, w2, tw, ti, **how)
+    ref = torch.cat([flag_gems.fused_experts_impl(x[b:b + 100].contiguous(), w1, w2, tw[b:b + 100], ti[b:b + 100], **how)
+                     for b in range(0, t, 100)])
+    assert torch.isfinite(out).all() and out.float().abs().max() > 0
+    assert torch.equal(out, ref)
