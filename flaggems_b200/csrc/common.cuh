@@ -119,27 +119,37 @@ void fg_count_launch(int n);
 __device__ __forceinline__ void fg_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void fg_pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// Launches `kernel` that way, with clusters of `cluster` CTAs when cluster > 1.
+// Launches `kernel` that way (or, without `early`, after everything before it), with clusters of `cluster` CTAs
+// when cluster > 1.
 template <typename... Params, typename... Args>
-cudaError_t fg_launch(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, unsigned cluster,
-                      Args&&... args) {
+cudaError_t fg_launch_when(bool early, void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
+                           unsigned cluster, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid, 1, 1);
     cfg.blockDim = dim3(block, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = cluster;
-    attr[1].val.clusterDim.y = 1;
-    attr[1].val.clusterDim.z = 1;
+    if (early) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = cluster;
+        attr[cfg.numAttrs].val.clusterDim.y = 1;
+        attr[cfg.numAttrs++].val.clusterDim.z = 1;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = cluster > 1 ? 2 : 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
     if (e == cudaSuccess) fg_count_launch(1);
     return e;
+}
+
+template <typename... Params, typename... Args>
+cudaError_t fg_launch(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, unsigned cluster,
+                      Args&&... args) {
+    return fg_launch_when(true, kernel, grid, block, smem, st, cluster, args...);
 }
 
 template <typename T> struct FgVec8;  // eight elements of T as raw words

@@ -1241,6 +1241,12 @@ int launch_splitk(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams
     return FG_OK;
 }
 
+// Whether a product is launched while its predecessor drains.  That saves ~2 us, but the CTAs then land on the
+// SMs in the order in which these fall free instead of by index, neighbouring tiles lose their common
+// die, and a long product draws more power for the same work: 4096 x 18432 x 7168 606 us launched early, 592 after.
+// Two waves of tiles take 20-100 us.
+bool short_run(int64_t tiles) { return tiles <= 2 * (int64_t)fg_num_sms(); }
+
 // CTA-pair kernel: clusters of two, one cluster per 256 x 256 tile, persistent over the tiles.
 // No block scales: with block scales the accumulator of every K block has to make the round
 // trip MMA -> both CTAs' epilogues -> MMA through cluster-wide barriers, and that latency costs
@@ -1274,7 +1280,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& 
         max_clusters = n < fg_num_sms() / 2 ? n : fg_num_sms() / 2;
     }
     const int clusters = pair_tiles < max_clusters ? pair_tiles : max_clusters;
-    FG_CUDA(fg_launch(kernel, (unsigned)(2 * clusters), C::THREADS, C::SMEM_BYTES, st, 2, ta, tb, p));
+    FG_CUDA(fg_launch_when(false, kernel, (unsigned)(2 * clusters), C::THREADS, C::SMEM_BYTES, st, 2, ta, tb, p));
     return FG_OK;
 }
 
@@ -1305,7 +1311,7 @@ int launch_inst(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& 
     int grid = fg_num_sms();
     if (max_tiles < grid) grid = max_tiles;
     if (grid < 1) grid = 1;
-    FG_CUDA(fg_launch(kernel, (unsigned)grid, C::THREADS, C::SMEM_BYTES, st, 1, ta, tb, p));
+    FG_CUDA(fg_launch_when(short_run(max_tiles), kernel, (unsigned)grid, C::THREADS, C::SMEM_BYTES, st, 1, ta, tb, p));
     return FG_OK;
 }
 
