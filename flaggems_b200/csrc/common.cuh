@@ -149,7 +149,10 @@ cudaError_t fg_launch_when(bool early, void (*kernel)(Params...), unsigned grid,
 template <typename... Params, typename... Args>
 cudaError_t fg_launch(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, unsigned cluster,
                       Args&&... args) {
-    return fg_launch_when(true, kernel, grid, block, smem, st, cluster, args...);
+    // Not where the grid fills more than half of the chip's thread slots: its CTAs would sit in them, waiting, while
+    // another stream (a layer's shared expert) has work for the SMs.
+    const bool early = (int64_t)grid * block <= 1024 * (int64_t)fg_num_sms();
+    return fg_launch_when(early, kernel, grid, block, smem, st, cluster, args...);
 }
 
 template <typename T> struct FgVec8;  // eight elements of T as raw words
