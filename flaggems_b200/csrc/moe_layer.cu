@@ -6,11 +6,12 @@
 //   gathered  (few rows per expert: decode) the GEMMs fetch their A rows through sorted_ids with
 //             tile::gather4 and store in route-slot order: nothing touches padding rows.  The copy into
 //             expert order and the padding cost 60 us of a 32-token DeepSeek-V3 step.
-//   sorted    (otherwise) rows are laid out in expert order, padded to 128 per expert, and fetched as
-//             TMA boxes.  Padding rows are zeros all the way: written once, they cost less than the tensor
-//             power that stale bytes in their place draw (2 % of a step under the power cap).  A gather4 of four 128-byte rows takes ~70 cycles whatever the rows, so a full tile
-//             of them (32 per K block) is four times slower than its MMAs: the line lies at 32 rows per
-//             expert, where eight lanes' gathers still hide behind the weight stream.
+//   sorted    (otherwise) rows are laid out in expert order, padded to 128 per expert (256 where CTA pairs run
+//             the products), and fetched as TMA boxes.  Padding rows are zeros all the way: written once,
+//             they cost less than the tensor power that stale bytes in their place draw (2 % of a step
+//             under the power cap).  A gather4 of four 128-byte rows takes ~70 cycles whatever the rows, so
+//             a full tile of them (32 per K block) is four times slower than its MMAs: the line lies
+//             where eight lanes' gathers still hide behind the weight stream (use_gather).
 #include <mutex>
 
 #include "common.cuh"
@@ -114,8 +115,11 @@ bool use_pairs(int64_t slots, int num_experts, int64_t n1, int64_t n2) {
     return slots >= PAIR_MIN_ROWS * (int64_t)num_experts && slots / PAIR_ROWS * (n / 256) >= 3 * (int64_t)(fg_num_sms() / 2);
 }
 
-// The line between the two row orders (see the head of this file).
-bool use_gather(int64_t slots, int num_experts) { return slots <= 32 * (int64_t)num_experts; }
+// The line between the two row orders (see the head of this file): 32 rows per expert, or 16 where the experts are
+// many.  A large router is skewed, and its popular experts then have full tiles of gathered rows long before
+// the average says so.  Gathered / sorted, us per step: DeepSeek-V3 (256 experts) 12 rows per expert
+// 2048 / 2101, 28 rows 2485 / 2356; Mixtral (8) 12 rows 260 / 280, 30 rows 277 / 282.
+bool use_gather(int64_t slots, int num_experts) { return slots <= (num_experts > 32 ? 16 : 32) * (int64_t)num_experts; }
 
 // Rows of one GEMM's input in the operand type of the mode; *scale is where their scales are.  `slots` (NULL or the
 // alignment table): only the rows that it names count toward a dynamic per-tensor scale.  In route-slot
