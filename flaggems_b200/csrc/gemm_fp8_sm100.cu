@@ -420,8 +420,10 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
         // Gathered A rows (few per tile, see the callers) are fetched by the whole warp: lane l names rows 4l .. 4l + 3 of the tile to one
         // tile::gather4, and lanes whose four rows are all padding fetch nothing (their rows of the
         // stage keep old bytes, which only reach accumulator rows nobody reads).
-        const bool gather = p.gather_div > 0 && !p.a_contiguous;
-        if (lane == 0 || gather) {
+        // Boxes are fetched by one lane, in a loop of its own: sharing the gathering loop cost block-scaled
+        // 4096 x 18432 x 7168 5 us of 597.
+        auto produce = [&](auto gather_tag) {
+            constexpr bool gather = decltype(gather_tag)::value;
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -432,11 +434,11 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                 if (expert < 0) continue;
                 int m0 = tc.m_blk * a_rows_step + (int)cta_rank * BLOCK_M;
                 const int n0 = tc.n_blk * OUT_TILE_N;
-                if (p.a_contiguous) m0 = p.sorted_ids[m0];
+                if (!gather && p.a_contiguous) m0 = p.sorted_ids[m0];
                 int4 rows = make_int4(0, 0, 0, 0);
                 bool mine = false;
                 uint32_t tx = stage_tx;
-                if (gather) {
+                if constexpr (gather) {
                     const int4 sid = *reinterpret_cast<const int4*>(p.sorted_ids + m0 + 4 * lane);
                     auto token = [&](int s) {
                         const bool real = s >= 0 && s < p.numel;
@@ -449,7 +451,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                 for (int kb = kb_begin; kb < kb_end; ++kb) {
                     FG_PROF_T0(tw);
                     ok = mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, 1);
-                    if (gather) ok = __all_sync(0xffffffffu, ok);
+                    if constexpr (gather) ok = __all_sync(0xffffffffu, ok);
                     FG_PROF_ADD(prof_wait, tw);
                     if (!ok) break;
                     uint8_t* sa = smem + stage * C::STAGE_BYTES;
@@ -471,7 +473,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                     }
                     if (lane == 0) {
                         mbar_arrive_expect_tx(&full_bar[stage], tx);
-                        if (!gather) tma_load_2d(sa, &tm_a, &full_bar[stage], kb * BLOCK_K, m0);
+                        if constexpr (!gather) tma_load_2d(sa, &tm_a, &full_bar[stage], kb * BLOCK_K, m0);
                         if constexpr (FUSE_SILU) {
                             tma_load_3d(sb, &tm_b, &full_bar[stage], kb * BLOCK_K, n0, expert);
                             tma_load_3d(sb + (BN / 2) * BLOCK_K, &tm_b, &full_bar[stage], kb * BLOCK_K, p.N / 2 + n0,
@@ -480,7 +482,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                             tma_load_3d(sb, &tm_b, &full_bar[stage], kb * BLOCK_K, n0, expert);
                         }
                     }
-                    if (gather) {
+                    if constexpr (gather) {
                         __syncwarp();
                         if (mine) tma_gather4(sa + lane * 4 * BLOCK_K, &tm_a, &full_bar[stage], kb * BLOCK_K, rows);
                     }
@@ -491,6 +493,12 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                 }
             }
             FG_PROF_OUT(0, prof_wait);
+        };
+        if constexpr (!PAIR) {
+            if (p.gather_div > 0 && !p.a_contiguous) produce(std::true_type());
+            else if (lane == 0) produce(std::false_type());
+        } else if (lane == 0) {
+            produce(std::false_type());
         }
         fg_pdl_trigger();  // every load of this CTA has been issued: only its last tile's epilogue is left
     } else if (ASTORE && warp == 3) {
