@@ -216,3 +216,23 @@ torch.testing.assert_close(c.cpu().float(), ref.float(), rtol=1e-2, atol=1e-2)
 
 def test_no_device_errors_recorded():
     assert _cabi.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("index", [[99, 5, 2, 99], [5, 99, 0, 3]])
+def test_per_tensor_dynamic_scale_with_padding_rows(index, dtype):
+    # the scale is written whichever rows are padding, the first among them
+    g = torch.Generator().manual_seed(7)
+    x = (torch.randn(3, 272, generator=g) * 3).to(dtype)
+    idx = torch.tensor(index, dtype=torch.int32).cuda()
+    amax = x.abs().amax().float().reshape(1).cuda()
+    scale = torch.full((1,), -1.0, device="cuda")
+    q = torch.full((4, 272), 0x55, dtype=U8, device="cuda")
+    xd = x.cuda()
+    _cabi.check(_cabi.lib().fg_per_tensor_quant_fp8(
+        _cabi.ptr(xd), _cabi.DTYPE_CODE[dtype], _cabi.ptr(q), _cabi.ptr(amax), 1, _cabi.ptr(scale), 4, 272, 272, 272,
+        _cabi.ptr(idx), 2, 6, None, _cabi.stream_ptr()))
+    qr, sr = oracle.per_tensor_quant_fp8(x)
+    assert torch.equal(_bits(scale.cpu()), _bits(sr.reshape(1)))
+    want = torch.stack([qr.view(U8)[i // 2] if i < 6 else torch.zeros(272, dtype=U8) for i in index])
+    _assert_bytes_equal(q, want)
