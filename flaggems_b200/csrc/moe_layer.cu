@@ -247,8 +247,12 @@ extern "C" {
 
 int64_t fg_scaled_grouped_mm_workspace_bytes(int64_t m_total, int num_groups, int64_t K) {
     if (m_total < 0 || num_groups <= 0 || K <= 0) return -1;
-    // the larger of the tables that the call may choose: its N is not known here
-    return carve_grouped_mm(nullptr, m_total, num_groups, m_total >= PAIR_MIN_ROWS * (int64_t)num_groups ? PAIR_ROWS : TILE_ROWS).bytes;
+    // The larger of the tables that the call may choose: its N is not known here.  Tables of 256-row blocks hold more
+    // padding, those of 128-row blocks more block ids (the larger part above ~32768 rows per group).
+    const int64_t single = carve_grouped_mm(nullptr, m_total, num_groups, TILE_ROWS).bytes;
+    if (m_total < PAIR_MIN_ROWS * (int64_t)num_groups) return single;
+    const int64_t paired = carve_grouped_mm(nullptr, m_total, num_groups, PAIR_ROWS).bytes;
+    return single > paired ? single : paired;
 }
 
 int fg_scaled_grouped_mm_fp8(void* c, const void* a, const void* b, const float* scale_a, const float* scale_b,

@@ -400,3 +400,16 @@ def test_scaled_grouped_mm_cta_pairs(offs):
             # fp32 sums of k products and one rounding to bf16
             torch.testing.assert_close(out[lo:hi].double(), ref, rtol=2 ** -8, atol=1e-5 * k)
         lo = hi
+
+
+def test_scaled_grouped_mm_many_rows_narrow_output():
+    # 65536 rows in one group, N = 128: 128-row blocks, whose tables are larger here than those of CTA pairs
+    g = torch.Generator(device="cuda").manual_seed(3)
+    m, n, k = 65536, 128, 64
+    a = torch.randn(m, k, device="cuda", generator=g).to(torch.float8_e4m3fn)
+    b = torch.randn(1, n, k, device="cuda", generator=g).to(torch.float8_e4m3fn)
+    sa, sb = torch.rand(m, device="cuda", generator=g), torch.rand(1, n, device="cuda", generator=g)
+    out = flag_gems.scaled_grouped_mm(a, b.transpose(1, 2), sa, sb, torch.tensor([m], dtype=torch.int32, device="cuda"))
+    ref = (a.double() @ b[0].double().t()) * sa[:, None].double() * sb[0].double()
+    # fp32 sums of k products and one rounding to bf16
+    torch.testing.assert_close(out.double(), ref, rtol=2 ** -8, atol=1e-5 * k)
