@@ -214,15 +214,15 @@ __global__ void __launch_bounds__(256) group_quant_kernel(QuantArgs a) {
     }
 }
 
-// ---- the expert-parallel dispatch format, 16-bit inputs, groups of 128 -------------------------------
-// Scales and a trailer sit behind the payload of each row, and rows are optionally stored into peers'
-// receive buffers.  A lane owns 16 consecutive elements (two 16-byte loads, one 16-byte store), kept as
-// raw 16-bit pairs; a team of eight lanes owns a group.
-template <typename T, int MODE>
-__global__ void __launch_bounds__(256, 5) group_pack16_kernel(QuantArgs a) {
+// ---- 16-bit inputs, a grid-stride loop over groups: rows that do not fill a CTA of their own, and the
+// expert-parallel dispatch format.  A lane owns 16 consecutive elements (two 16-byte loads, one 16-byte store),
+// kept as raw 16-bit pairs; a team of GROUP/16 lanes owns a group.  PACKED: scales and a trailer sit behind
+// the payload of each row, and rows are optionally stored into peers' receive buffers.
+template <typename T, int MODE, int TPG, bool PACKED>
+__global__ void __launch_bounds__(256, 5) group_quant16_kernel(QuantArgs a) {
     fg_pdl_wait();
     fg_pdl_trigger();
-    constexpr int UNROLL = 2, TPG = 8;
+    constexpr int UNROLL = 2;
     constexpr int GROUP = TPG * 16;
     using P = Pair16<T>;
     const int64_t rows = resolve_rows(a);
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(256, 5) group_pack16_kernel(QuantArgs a) {
             const float s = make_scale<MODE>(amax, a.eps, a.pow2);
             const Divider d = make_divider<MODE>(s);
             uint8_t* qrow = nullptr;
-            if (row[u] < rows) qrow = packed_row_ptr(a, row[u]);
+            if (row[u] < rows) qrow = PACKED ? packed_row_ptr(a, row[u]) : a.q + (int64_t)row[u] * a.ld_q;
             if (qrow) {
                 uint32_t o[4];
 #pragma unroll
@@ -285,8 +285,12 @@ __global__ void __launch_bounds__(256, 5) group_pack16_kernel(QuantArgs a) {
                 }
                 *reinterpret_cast<uint4*>(qrow + cg[u] * GROUP + lane_in_team * 16) = make_uint4(o[0], o[1], o[2], o[3]);
                 if (lane_in_team == 0) {
-                    reinterpret_cast<float*>(qrow + a.K)[cg[u]] = s;
-                    if (cg[u] == 0) write_row_meta(a, row[u]);
+                    if constexpr (PACKED) {  // scales sit behind the payload of the same row
+                        reinterpret_cast<float*>(qrow + a.K)[cg[u]] = s;
+                        if (cg[u] == 0) write_row_meta(a, row[u]);
+                    } else {
+                        a.s[(int64_t)row[u] * a.s_row_stride + (int64_t)cg[u] * a.s_col_stride] = s;
+                    }
                 }
             }
             cg[u] += step_cg;
@@ -615,6 +619,17 @@ __global__ void __launch_bounds__(256) abs_max_kernel(const T* __restrict__ x, i
     }
 }
 
+// Whether rows in groups get a CTA each (group_row16_kernel) or share CTAs in the loop of group_quant16_kernel.  The
+// chip starts one small CTA per ~1.03 ns, whatever its row holds: 65536 rows of 128 take 68 us a CTA each and 7.0 in
+// the loop, 65536 x 1536 68 and 56; from 1920 elements on a row's own bytes take longer than its start
+// (52429 x 1920 55 and 56, 49152 x 2048 51 and 56).  Few rows are started in less time than the loop's index
+// arithmetic takes: 512 x 128 1.8 and 2.6 us, 2048 x 512 2.7 and 2.8 (3072 rows: 3.7 and 3.1), 4096 x 1024 4.9 both
+// (8192 rows: 9.2 and 6.9).  A CTA holds up to 32768 elements.
+bool use_row_ctas(int64_t rows, int64_t K) {
+    if (K > 1024 * 16 * ROW_UNITS || rows >= (1ll << 31)) return false;
+    return K >= 1920 || rows <= (4 * K > 2048 ? 4 * K : 2048);
+}
+
 template <typename T, int MODE>
 int launch_quant_t(const QuantArgs& a, cudaStream_t st) {
     if (a.rows == 0 || a.K == 0) return FG_OK;
@@ -630,20 +645,22 @@ int launch_quant_t(const QuantArgs& a, cudaStream_t st) {
     };
     if constexpr (sizeof(T) == 2) {
         const int64_t threads = fg_cdiv(fg_cdiv(a.K, 16 * ROW_UNITS), 32) * 32;
-        auto by_row = [&](auto kernel) -> int {
-            FG_CUDA(fg_launch(kernel, (unsigned)a.rows, (unsigned)threads, 0, st, 1, a));
-            return FG_OK;
-        };
         // 16-byte stores need 16-byte aligned output rows; otherwise the generic kernel below
         const bool q16 = ((uintptr_t)a.q % 16 == 0) && (a.ld_q % 16 == 0);
+        auto by_group = [&](auto tpg) -> int {
+            constexpr int TPG = decltype(tpg)::value;
+            if (!use_row_ctas(a.rows, a.K)) return small(group_quant16_kernel<T, MODE, TPG, false>, TPG);
+            FG_CUDA(fg_launch(group_row16_kernel<T, MODE, TPG>, (unsigned)a.rows, (unsigned)threads, 0, st, 1, a));
+            return FG_OK;
+        };
         if (q16 && a.meta_ids) {
-            if (a.group == 128) return small(group_pack16_kernel<T, MODE>, 8);
-        } else if (q16 && threads <= 1024 && a.rows < (1ll << 31)) {
+            if (a.group == 128) return small(group_quant16_kernel<T, MODE, 8, true>, 8);
+        } else if (q16) {
             switch (a.group) {
-                case 64: return by_row(group_row16_kernel<T, MODE, 4>);
-                case 128: return by_row(group_row16_kernel<T, MODE, 8>);
-                case 256: return by_row(group_row16_kernel<T, MODE, 16>);
-                case 512: return by_row(group_row16_kernel<T, MODE, 32>);
+                case 64: return by_group(std::integral_constant<int, 4>());
+                case 128: return by_group(std::integral_constant<int, 8>());
+                case 256: return by_group(std::integral_constant<int, 16>());
+                case 512: return by_group(std::integral_constant<int, 32>());
                 default: break;
             }
         }
