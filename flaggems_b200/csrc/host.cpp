@@ -120,6 +120,18 @@ PyObject* pair(at::Tensor a, at::Tensor b) {
     return t;
 }
 
+// Runs f without the interpreter lock, as ctypes does: allocations and launches may block (a full launch queue, an
+// allocation that frees cached blocks, a kernel's first load), and the thread that they wait for may be a Python one.
+// The operands belong to the caller's frame, which keeps them alive.
+template <typename F>
+auto unlocked(F&& f) {
+    struct Released {
+        PyThreadState* state = PyEval_SaveThread();
+        ~Released() { PyEval_RestoreThread(state); }
+    } released;
+    return f();
+}
+
 // C++ exceptions (an allocation that fails) become Python ones.
 template <typename F>
 PyObject* guarded(F&& f) {
@@ -148,14 +160,18 @@ PyObject* group_quant(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (!x || dtype_code(x->scalar_type()) < 0 || !as_rows(*x, &m, &k, &ld) || k % group) return none();
         const bool column = PyObject_IsTrue(a[3]) == 1, ue8m0 = PyObject_IsTrue(a[4]) == 1;
         if (column && x->dim() != 2) return none();
-        c10::cuda::CUDAGuard guard(x->device());
+        const float eps = (float)PyFloat_AS_DOUBLE(a[2]);
         const int64_t g = k / group;
-        at::Tensor q = empty(x->sizes(), E4M3, *x);
-        at::Tensor s = column ? at::Tensor(at::detail::empty_strided_cuda({m, g}, {1, m}, ScalarType::Float, x->device()))
-                              : empty(sizes_with_last(*x, g), ScalarType::Float, *x);
-        const int rc = fg_per_token_group_quant_fp8(
-            x->data_ptr(), dtype_code(x->scalar_type()), q.data_ptr(), static_cast<float*>(s.data_ptr()), m, k, (int)group,
-            ld, k, column ? 1 : g, column ? m : 1, (float)PyFloat_AS_DOUBLE(a[2]), ue8m0, stream_of(*x));
+        at::Tensor q, s;
+        const int rc = unlocked([&] {
+            c10::cuda::CUDAGuard guard(x->device());
+            q = empty(x->sizes(), E4M3, *x);
+            s = column ? at::Tensor(at::detail::empty_strided_cuda({m, g}, {1, m}, ScalarType::Float, x->device()))
+                       : empty(sizes_with_last(*x, g), ScalarType::Float, *x);
+            return fg_per_token_group_quant_fp8(x->data_ptr(), dtype_code(x->scalar_type()), q.data_ptr(),
+                                                static_cast<float*>(s.data_ptr()), m, k, (int)group, ld, k, column ? 1 : g,
+                                                column ? m : 1, eps, ue8m0, stream_of(*x));
+        });
         if (rc != FG_OK) return raise_rc(rc);
         return pair(std::move(q), std::move(s));
     });
@@ -169,10 +185,15 @@ PyObject* act_quant(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const at::Tensor* x = cuda_tensor(a[0]);
         if (!x || x->scalar_type() != ScalarType::BFloat16 || !x->is_contiguous() || !as_rows(*x, &m, &k, &ld) || k % block)
             return none();
-        c10::cuda::CUDAGuard guard(x->device());
-        at::Tensor y = empty(x->sizes(), E4M3, *x), s = empty(sizes_with_last(*x, k / block), ScalarType::Float, *x);
-        const int rc = fg_act_quant_bf16_e4m3(x->data_ptr(), y.data_ptr(), static_cast<float*>(s.data_ptr()), m, k,
-                                              (int)block, k, k, k / block, PyObject_IsTrue(a[2]) == 1, stream_of(*x));
+        const bool pow2 = PyObject_IsTrue(a[2]) == 1;
+        at::Tensor y, s;
+        const int rc = unlocked([&] {
+            c10::cuda::CUDAGuard guard(x->device());
+            y = empty(x->sizes(), E4M3, *x);
+            s = empty(sizes_with_last(*x, k / block), ScalarType::Float, *x);
+            return fg_act_quant_bf16_e4m3(x->data_ptr(), y.data_ptr(), static_cast<float*>(s.data_ptr()), m, k, (int)block, k,
+                                          k, k / block, pow2, stream_of(*x));
+        });
         if (rc != FG_OK) return raise_rc(rc);
         return pair(std::move(y), std::move(s));
     });
@@ -184,11 +205,14 @@ PyObject* token_quant(PyObject*, PyObject* const* a, Py_ssize_t n) {
         int64_t m, k, ld;
         const at::Tensor* x = n == 1 ? cuda_tensor(a[0]) : nullptr;
         if (!x || dtype_code(x->scalar_type()) < 0 || !as_rows(*x, &m, &k, &ld)) return none();
-        c10::cuda::CUDAGuard guard(x->device());
-        at::Tensor q = empty(x->sizes(), E4M3, *x), s = empty(sizes_with_last(*x, 1), ScalarType::Float, *x);
-        const int rc = fg_per_token_quant_fp8(x->data_ptr(), dtype_code(x->scalar_type()), q.data_ptr(),
-                                              static_cast<float*>(s.data_ptr()), m, k, ld, k, nullptr, 1, 0, nullptr,
-                                              stream_of(*x));
+        at::Tensor q, s;
+        const int rc = unlocked([&] {
+            c10::cuda::CUDAGuard guard(x->device());
+            q = empty(x->sizes(), E4M3, *x);
+            s = empty(sizes_with_last(*x, 1), ScalarType::Float, *x);
+            return fg_per_token_quant_fp8(x->data_ptr(), dtype_code(x->scalar_type()), q.data_ptr(),
+                                          static_cast<float*>(s.data_ptr()), m, k, ld, k, nullptr, 1, 0, nullptr, stream_of(*x));
+        });
         if (rc != FG_OK) return raise_rc(rc);
         return pair(std::move(q), std::move(s));
     });
@@ -203,11 +227,14 @@ PyObject* tensor_quant(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (!s || s->scalar_type() != ScalarType::Float || s->numel() < 1 || dtype_code(x->scalar_type()) < 0 ||
             !as_rows(*x, &m, &k, &ld))
             return none();
-        c10::cuda::CUDAGuard guard(x->device());
-        at::Tensor q = empty(x->sizes(), E4M3, *x);
-        float* scale = static_cast<float*>(s->data_ptr());
-        const int rc = fg_per_tensor_quant_fp8(x->data_ptr(), dtype_code(x->scalar_type()), q.data_ptr(), scale, 0, scale, m,
-                                               k, ld, k, nullptr, 1, 0, nullptr, stream_of(*x));
+        at::Tensor q;
+        const int rc = unlocked([&] {
+            c10::cuda::CUDAGuard guard(x->device());
+            q = empty(x->sizes(), E4M3, *x);
+            float* scale = static_cast<float*>(s->data_ptr());
+            return fg_per_tensor_quant_fp8(x->data_ptr(), dtype_code(x->scalar_type()), q.data_ptr(), scale, 0, scale, m, k, ld,
+                                           k, nullptr, 1, 0, nullptr, stream_of(*x));
+        });
         if (rc != FG_OK) return raise_rc(rc);
         return THPVariable_Wrap(std::move(q));
     });
@@ -244,12 +271,14 @@ PyObject* block_mm(PyObject*, PyObject* const* a, Py_ssize_t n) {
         } else if (!As->is_contiguous()) {
             return none();
         }
-        c10::cuda::CUDAGuard guard(A->device());
-        at::Tensor c = empty(sizes_with_last(*A, rows_b), out, *A);
-        const int rc = fg_block_scaled_mm_fp8(c.data_ptr(), A->data_ptr(), B->data_ptr(),
-                                              static_cast<const float*>(As->data_ptr()),
-                                              static_cast<const float*>(Bs->data_ptr()), m, rows_b, k, k, B->stride(0), rows_b,
-                                              as_row, as_col, Bs->stride(0), Bs->stride(1), dtype_code(out), stream_of(*A));
+        at::Tensor c;
+        const int rc = unlocked([&] {
+            c10::cuda::CUDAGuard guard(A->device());
+            c = empty(sizes_with_last(*A, rows_b), out, *A);
+            return fg_block_scaled_mm_fp8(c.data_ptr(), A->data_ptr(), B->data_ptr(), static_cast<const float*>(As->data_ptr()),
+                                          static_cast<const float*>(Bs->data_ptr()), m, rows_b, k, k, B->stride(0), rows_b,
+                                          as_row, as_col, Bs->stride(0), Bs->stride(1), dtype_code(out), stream_of(*A));
+        });
         if (rc != FG_OK) return raise_rc(rc);
         return THPVariable_Wrap(std::move(c));
     });
@@ -287,12 +316,13 @@ PyObject* scaled_mm(PyObject*, PyObject* const* p, Py_ssize_t n) {
             const ScalarType want = code == FG_DTYPE_E4M3 ? ScalarType::Float : c->scalar_type();
             if (!bias || bias->scalar_type() != want || bias->dim() != 1 || bias->size(0) != cols || !bias->is_contiguous()) return none();
         }
-        c10::cuda::CUDAGuard guard(a->device());
-        const int rc = fg_scaled_mm_fp8(
-            c->data_ptr(), a->data_ptr(), b->data_ptr(), static_cast<const float*>(sa->data_ptr()),
-            static_cast<const float*>(sb->data_ptr()), bias ? bias->data_ptr() : nullptr, m, cols, k, a->stride(0), b->stride(1),
-            c->stride(0), sa->numel() > 1 ? FG_SCALE_VECTOR : FG_SCALE_SCALAR,
-            sb->numel() > 1 ? FG_SCALE_VECTOR : FG_SCALE_SCALAR, code, cutlass, stream_of(*a));
+        const int rc = unlocked([&] {
+            c10::cuda::CUDAGuard guard(a->device());
+            return fg_scaled_mm_fp8(c->data_ptr(), a->data_ptr(), b->data_ptr(), static_cast<const float*>(sa->data_ptr()),
+                                    static_cast<const float*>(sb->data_ptr()), bias ? bias->data_ptr() : nullptr, m, cols, k,
+                                    a->stride(0), b->stride(1), c->stride(0), sa->numel() > 1 ? FG_SCALE_VECTOR : FG_SCALE_SCALAR,
+                                    sb->numel() > 1 ? FG_SCALE_VECTOR : FG_SCALE_SCALAR, code, cutlass, stream_of(*a));
+        });
         if (rc != FG_OK) return raise_rc(rc);
         Py_INCREF(p[0]);
         return p[0];
@@ -306,7 +336,7 @@ PyObject* scaled_mm_new(PyObject* self, PyObject* const* p, Py_ssize_t n) {
         const at::Tensor *a = n == 6 ? cuda_tensor(p[0]) : nullptr, *b = a ? cuda_tensor(p[1]) : nullptr;
         if (!b || a->dim() != 2 || b->dim() != 2 || !py_dtype(p[5], &out) || (out != E4M3 && dtype_code(out) < 0)) return none();
         if (a->size(0) == 0 || b->size(1) == 0) return none();
-        PyObject* c = THPVariable_Wrap(empty({a->size(0), b->size(1)}, out, *a));
+        PyObject* c = THPVariable_Wrap(unlocked([&] { return empty({a->size(0), b->size(1)}, out, *a); }));
         if (!c) return nullptr;
         PyObject* args[7] = {c, p[0], p[1], p[2], p[3], p[4], Py_False};
         PyObject* r = scaled_mm(self, args, 7);
@@ -332,14 +362,17 @@ PyObject* grouped_mm(PyObject*, PyObject* const* p, Py_ssize_t n) {
             sb->scalar_type() != ScalarType::Float || sb->size(0) != groups || sb->size(1) != cols || !sb->is_contiguous() ||
             offs->scalar_type() != ScalarType::Int || offs->size(0) != groups || !offs->is_contiguous())
             return none();
-        c10::cuda::CUDAGuard guard(a->device());
-        at::Tensor c = empty({m, cols}, out, *a);
-        const int64_t need = fg_scaled_grouped_mm_workspace_bytes(m, (int)groups, k) + 256;
-        at::Tensor ws = empty({need}, ScalarType::Byte, *a);
-        const int rc = fg_scaled_grouped_mm_fp8(
-            c.data_ptr(), a->data_ptr(), b->data_ptr(), static_cast<const float*>(sa->data_ptr()),
-            static_cast<const float*>(sb->data_ptr()), nullptr, 0, static_cast<const int32_t*>(offs->data_ptr()), (int)groups, m,
-            cols, k, a->stride(0), cols, dtype_code(out), ws.data_ptr(), need, stream_of(*a));
+        at::Tensor c, ws;
+        const int rc = unlocked([&] {
+            c10::cuda::CUDAGuard guard(a->device());
+            c = empty({m, cols}, out, *a);
+            const int64_t need = fg_scaled_grouped_mm_workspace_bytes(m, (int)groups, k) + 256;
+            ws = empty({need}, ScalarType::Byte, *a);
+            return fg_scaled_grouped_mm_fp8(c.data_ptr(), a->data_ptr(), b->data_ptr(), static_cast<const float*>(sa->data_ptr()),
+                                            static_cast<const float*>(sb->data_ptr()), nullptr, 0,
+                                            static_cast<const int32_t*>(offs->data_ptr()), (int)groups, m, cols, k, a->stride(0),
+                                            cols, dtype_code(out), ws.data_ptr(), need, stream_of(*a));
+        });
         if (rc != FG_OK) return raise_rc(rc);
         return THPVariable_Wrap(std::move(c));
     });
@@ -360,10 +393,13 @@ PyObject* topk_softmax(PyObject*, PyObject* const* p, Py_ssize_t n) {
         const ScalarType it = idx->scalar_type();
         const int kind = it == ScalarType::Int ? 0 : it == ScalarType::UInt32 ? 1 : it == ScalarType::Long ? 2 : -1;
         if (kind < 0 || dtype_code(g->scalar_type()) < 0) return none();
-        c10::cuda::CUDAGuard guard(g->device());
-        const int rc = fg_topk_softmax(static_cast<float*>(w->data_ptr()), idx->data_ptr(), kind,
-                                       static_cast<int32_t*>(src->data_ptr()), g->data_ptr(), dtype_code(g->scalar_type()), t,
-                                       (int)e, (int)k, PyObject_IsTrue(p[4]) == 1, nullptr, stream_of(*g));
+        const bool renormalize = PyObject_IsTrue(p[4]) == 1;
+        const int rc = unlocked([&] {
+            c10::cuda::CUDAGuard guard(g->device());
+            return fg_topk_softmax(static_cast<float*>(w->data_ptr()), idx->data_ptr(), kind, static_cast<int32_t*>(src->data_ptr()),
+                                   g->data_ptr(), dtype_code(g->scalar_type()), t, (int)e, (int)k, renormalize, nullptr,
+                                   stream_of(*g));
+        });
         if (rc != FG_OK) return raise_rc(rc);
         Py_RETURN_TRUE;
     });
@@ -382,12 +418,17 @@ PyObject* grouped_topk(PyObject*, PyObject* const* p, Py_ssize_t n) {
         if (t == 0 || n_group < 1 || n_group > 32 || e % n_group || topk > 32 || (scoring != 0 && scoring != 1)) return none();
         if (s->stride(1) != 1 || bias->scalar_type() != s->scalar_type() || bias->size(0) != e || !bias->is_contiguous())
             return none();
-        c10::cuda::CUDAGuard guard(s->device());
-        at::Tensor w = empty({t, topk}, ScalarType::Float, *s), idx = empty({t, topk}, ScalarType::Int, *s);
-        const int rc = fg_grouped_topk(static_cast<float*>(w.data_ptr()), static_cast<int32_t*>(idx.data_ptr()), s->data_ptr(),
-                                       bias->data_ptr(), dtype_code(s->scalar_type()), t, (int)e, s->stride(0), (int)n_group,
-                                       (int)topk_group, (int)topk, PyObject_IsTrue(p[4]) == 1, (float)PyFloat_AS_DOUBLE(p[5]),
-                                       (int)scoring, nullptr, stream_of(*s));
+        const bool renormalize = PyObject_IsTrue(p[4]) == 1;
+        const float scaling = (float)PyFloat_AS_DOUBLE(p[5]);
+        at::Tensor w, idx;
+        const int rc = unlocked([&] {
+            c10::cuda::CUDAGuard guard(s->device());
+            w = empty({t, topk}, ScalarType::Float, *s);
+            idx = empty({t, topk}, ScalarType::Int, *s);
+            return fg_grouped_topk(static_cast<float*>(w.data_ptr()), static_cast<int32_t*>(idx.data_ptr()), s->data_ptr(),
+                                   bias->data_ptr(), dtype_code(s->scalar_type()), t, (int)e, s->stride(0), (int)n_group,
+                                   (int)topk_group, (int)topk, renormalize, scaling, (int)scoring, nullptr, stream_of(*s));
+        });
         if (rc != FG_OK) return raise_rc(rc);
         return pair(std::move(w), std::move(idx));
     });
@@ -402,13 +443,16 @@ PyObject* moe_align(PyObject*, PyObject* const* p, Py_ssize_t n) {
             return none();
         const bool i64 = ids->scalar_type() == ScalarType::Long;
         if (!i64 && ids->scalar_type() != ScalarType::Int) return none();
-        c10::cuda::CUDAGuard guard(ids->device());
-        at::Tensor sorted = empty({pad}, ScalarType::Int, *ids), eids = empty({(pad + bs - 1) / bs}, ScalarType::Int, *ids),
-                   post = empty({1}, ScalarType::Int, *ids);
-        const int rc = fg_moe_align_block_size(ids->data_ptr(), i64, ids->numel(), (int)e, (int)bs, nullptr, 0,
-                                               static_cast<int32_t*>(sorted.data_ptr()), pad,
-                                               static_cast<int32_t*>(eids.data_ptr()), eids.numel(),
-                                               static_cast<int32_t*>(post.data_ptr()), stream_of(*ids));
+        at::Tensor sorted, eids, post;
+        const int rc = unlocked([&] {
+            c10::cuda::CUDAGuard guard(ids->device());
+            sorted = empty({pad}, ScalarType::Int, *ids);
+            eids = empty({(pad + bs - 1) / bs}, ScalarType::Int, *ids);
+            post = empty({1}, ScalarType::Int, *ids);
+            return fg_moe_align_block_size(ids->data_ptr(), i64, ids->numel(), (int)e, (int)bs, nullptr, 0,
+                                           static_cast<int32_t*>(sorted.data_ptr()), pad, static_cast<int32_t*>(eids.data_ptr()),
+                                           eids.numel(), static_cast<int32_t*>(post.data_ptr()), stream_of(*ids));
+        });
         if (rc != FG_OK) return raise_rc(rc);
         PyObject* t = PyTuple_New(3);
         if (!t) return nullptr;
@@ -436,16 +480,18 @@ PyObject* silu_mul(PyObject*, PyObject* const* p, Py_ssize_t n) {
         at::Tensor made;
         const at::Tensor* o = nullptr;
         if (p[2] == Py_None) {
-            made = empty(x->sizes(), x->scalar_type(), *x);
+            made = unlocked([&] { return empty(x->sizes(), x->scalar_type(), *x); });
             o = &made;
         } else {
             o = cuda_tensor(p[2]);
             if (!o || o->sizes() != x->sizes() || o->scalar_type() != x->scalar_type()) return none();
         }
         if (!as_rows(*o, &m2, &k2, &ldo)) return none();
-        c10::cuda::CUDAGuard guard(x->device());
-        const int rc = fg_silu_and_mul(x->data_ptr(), y->data_ptr(), o->data_ptr(), m, k, ldx, ldy, ldo,
-                                       dtype_code(x->scalar_type()), stream_of(*x));
+        const int rc = unlocked([&] {
+            c10::cuda::CUDAGuard guard(x->device());
+            return fg_silu_and_mul(x->data_ptr(), y->data_ptr(), o->data_ptr(), m, k, ldx, ldy, ldo, dtype_code(x->scalar_type()),
+                                   stream_of(*x));
+        });
         if (rc != FG_OK) return raise_rc(rc);
         if (made.defined()) return THPVariable_Wrap(std::move(made));
         Py_INCREF(p[2]);
@@ -460,9 +506,11 @@ PyObject* moe_sum(PyObject*, PyObject* const* p, Py_ssize_t n) {
         if (!o || x->dim() != 3 || o->dim() != 2 || x->scalar_type() != o->scalar_type() || dtype_code(x->scalar_type()) < 0)
             return none();
         if (o->size(0) != x->size(0) || o->size(1) != x->size(2) || !x->is_contiguous() || !o->is_contiguous()) return none();
-        c10::cuda::CUDAGuard guard(x->device());
-        const int rc = fg_moe_sum(x->data_ptr(), o->data_ptr(), x->size(0), (int)x->size(1), x->size(2),
-                                  dtype_code(x->scalar_type()), stream_of(*x));
+        const int rc = unlocked([&] {
+            c10::cuda::CUDAGuard guard(x->device());
+            return fg_moe_sum(x->data_ptr(), o->data_ptr(), x->size(0), (int)x->size(1), x->size(2), dtype_code(x->scalar_type()),
+                              stream_of(*x));
+        });
         if (rc != FG_OK) return raise_rc(rc);
         Py_INCREF(p[1]);
         return p[1];
@@ -492,21 +540,26 @@ PyObject* fused_experts(PyObject*, PyObject* const* p, Py_ssize_t n) {
         if (experts < w1->size(0)) experts = w1->size(0);  // more weights than the count names: ids stay below it
         const int code = dtype_code(x->scalar_type()), esz = (int)x->element_size();
         const bool i64 = ids->scalar_type() == ScalarType::Long;
-        c10::cuda::CUDAGuard guard(x->device());
-        const int64_t most = t < chunk ? t : chunk;
-        const int64_t need = fg_fused_experts_workspace_bytes((int)mode, most, (int)topk, (int)experts, h, inter, code);
-        at::Tensor ws = empty({need}, ScalarType::Byte, *x);
-        for (int64_t b = 0; b < t; b += chunk) {
-            const int64_t rows = t - b < chunk ? t - b : chunk;
-            const int rc = fg_fused_experts(
-                static_cast<char*>(out->data_ptr()) + b * h * esz, static_cast<const char*>(x->data_ptr()) + b * h * esz, code,
-                static_cast<const char*>(ids->data_ptr()) + b * topk * (i64 ? 8 : 4), i64,
-                static_cast<const char*>(tw->data_ptr()) + b * topk * tw->element_size(), dtype_code(tw->scalar_type()), rows,
-                (int)topk, w1->data_ptr(), w2->data_ptr(), f[0], f[1], f[2], f[3], (int)mode, (int)experts, (int)w1->size(0),
-                map ? static_cast<const int32_t*>(map->data_ptr()) : nullptr, map ? (int)map->numel() : 0, h, inter, nullptr,
-                ws.data_ptr(), need, stream_of(*x));
-            if (rc != FG_OK) return raise_rc(rc);
-        }
+        at::Tensor ws;
+        const int rc = unlocked([&] {
+            c10::cuda::CUDAGuard guard(x->device());
+            const int64_t most = t < chunk ? t : chunk;
+            const int64_t need = fg_fused_experts_workspace_bytes((int)mode, most, (int)topk, (int)experts, h, inter, code);
+            ws = empty({need}, ScalarType::Byte, *x);
+            for (int64_t b = 0; b < t; b += chunk) {
+                const int64_t rows = t - b < chunk ? t - b : chunk;
+                const int e = fg_fused_experts(
+                    static_cast<char*>(out->data_ptr()) + b * h * esz, static_cast<const char*>(x->data_ptr()) + b * h * esz, code,
+                    static_cast<const char*>(ids->data_ptr()) + b * topk * (i64 ? 8 : 4), i64,
+                    static_cast<const char*>(tw->data_ptr()) + b * topk * tw->element_size(), dtype_code(tw->scalar_type()), rows,
+                    (int)topk, w1->data_ptr(), w2->data_ptr(), f[0], f[1], f[2], f[3], (int)mode, (int)experts, (int)w1->size(0),
+                    map ? static_cast<const int32_t*>(map->data_ptr()) : nullptr, map ? (int)map->numel() : 0, h, inter, nullptr,
+                    ws.data_ptr(), need, stream_of(*x));
+                if (e != FG_OK) return e;
+            }
+            return (int)FG_OK;
+        });
+        if (rc != FG_OK) return raise_rc(rc);
         Py_INCREF(p[5]);
         return p[5];
     });

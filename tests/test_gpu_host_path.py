@@ -1,5 +1,8 @@
 """The native host path and the Python code behind it give the same results for the same call, and the
 calls that the native path leaves alone still end in the Python code's errors."""
+import threading
+import time
+
 import pytest
 import torch
 
@@ -98,3 +101,31 @@ def test_refused_calls_still_raise():
         flag_gems.per_token_group_quant_fp8(_rand(1, 1025)[:, 1:], 128)
     with pytest.raises(AssertionError, match="must be divisible"):
         flag_gems.per_token_group_quant_fp8(_rand(1, 100), 128)
+
+
+def test_other_threads_run_while_a_call_blocks():
+    # A kernel of about 0.6 s in front of more launches than the queue holds: the calls block, other Python threads do not.
+    x = _rand(1, 256)
+    flag_gems.act_quant_triton(x, 128)
+    torch.cuda.synchronize()
+    ticks, stop = [], threading.Event()
+
+    def tick():
+        while not stop.is_set():
+            ticks.append(time.monotonic())
+            time.sleep(0.002)
+
+    thread = threading.Thread(target=tick)
+    thread.start()
+    try:
+        torch.cuda._sleep(1_200_000_000)  # GPU clocks, below 2 GHz
+        begin = time.monotonic()
+        for _ in range(6000):
+            flag_gems.act_quant_triton(x, 128)
+        blocked = time.monotonic() - begin
+    finally:
+        stop.set()
+        thread.join()
+    torch.cuda.synchronize()
+    assert blocked > 0.3, "the launch queue never filled: nothing was tested"
+    assert max(b - a for a, b in zip(ticks, ticks[1:])) < 0.15
