@@ -14,7 +14,6 @@ import torch
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "lib", "libflaggems_b200.so")
-HOST_PATH = os.path.join(_HERE, "lib", "_fg_host.so")
 
 FG_OK = 0
 DTYPE_CODE = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
@@ -140,9 +139,13 @@ class _NativeHost:
     Each returns None for a call that it leaves to the Python code behind it."""
 
     def __getattr__(self, name):
-        if not os.path.exists(HOST_PATH):
-            raise FlagGemsB200Error(f"{HOST_PATH} not found: build it with `python -m flaggems_b200.build`.")
-        loader = importlib.machinery.ExtensionFileLoader("_fg_host", HOST_PATH)
+        from .build import host_path
+
+        path = host_path()
+        if not os.path.exists(path):
+            raise FlagGemsB200Error(f"{path} (the host module for this Python and torch) not found: "
+                                    "build it with `python -m flaggems_b200.build`.")
+        loader = importlib.machinery.ExtensionFileLoader("_fg_host", path)
         module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_fg_host", loader))
         loader.exec_module(module)
         self.__dict__.update({k: v for k, v in vars(module).items() if not k.startswith("_")})

@@ -2,8 +2,8 @@
 
     python -m flaggems_b200.build [--force] [--verbose]
 
-Produces ``flaggems_b200/lib/libflaggems_b200.so`` and ``lib/_fg_host.so`` next to the sources
-(in-tree, git-ignored).  nvcc cross-compiles without a GPU.  No fast-math flags: the
+Produces ``flaggems_b200/lib/libflaggems_b200.so`` and ``lib/_fg_host.<python and torch>.so`` next to the
+sources (in-tree, git-ignored).  nvcc cross-compiles without a GPU.  No fast-math flags: the
 quantisation kernels rely on IEEE fp32 semantics.
 """
 import argparse
@@ -17,7 +17,6 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libflaggems_b200.so")
-HOST_PATH = os.path.join(LIB_DIR, "_fg_host.so")
 SOURCES = ["api.cu", "quant.cu", "moe_glue.cu", "moe_layer.cu", "router.cu", "gemm_fp8_sm100.cu"]
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
@@ -37,10 +36,19 @@ def _stale(path, sources):
     return any(os.path.getmtime(d) > os.path.getmtime(path) for d in deps)
 
 
+def host_path():
+    """File of the native host module for the running Python and torch: it is bound to the C++ interfaces of both,
+    so another version of either needs a module of its own."""
+    import torch
+
+    return os.path.join(LIB_DIR, f"_fg_host.{sysconfig.get_config_var('SOABI')}.torch-{torch.__version__}"
+                                 f".abi{int(torch._C._GLIBCXX_USE_CXX11_ABI)}.so")
+
+
 def build(force=False, verbose=False):
     if force or _stale(LIB_PATH, [f for f in os.listdir(CSRC) if f != "host.cpp"]):
         build_library(verbose)
-    if force or _stale(HOST_PATH, ["host.cpp"]):
+    if force or _stale(host_path(), ["host.cpp"]):
         build_host()
     return LIB_PATH
 
@@ -55,7 +63,7 @@ def build_host():
     cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            f"-I{os.path.join(root, 'include')}", f"-I{os.path.join(root, 'include', 'torch', 'csrc', 'api', 'include')}",
            f"-I{os.path.join(cuda, 'include')}", f"-I{sysconfig.get_paths()['include']}",
-           os.path.join(CSRC, "host.cpp"), "-o", HOST_PATH, f"-L{os.path.join(root, 'lib')}",
+           os.path.join(CSRC, "host.cpp"), "-o", host_path(), f"-L{os.path.join(root, 'lib')}",
            "-ltorch", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10", "-lc10_cuda",
            f"-L{LIB_DIR}", "-lflaggems_b200", "-Wl,-rpath,$ORIGIN"]
     r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)

@@ -54,3 +54,23 @@ def test_missing_library_fails_loudly(monkeypatch):
     monkeypatch.setattr(_cabi, "LIB_PATH", "/nonexistent/libflaggems_b200.so")
     with pytest.raises(_cabi.FlagGemsB200Error):
         _cabi.lib()
+
+
+def test_another_torch_gets_a_host_module_of_its_own(monkeypatch):
+    import torch
+
+    from flaggems_b200 import _cabi
+    from flaggems_b200 import build as b
+
+    made = []
+    b.build()
+    monkeypatch.setattr(b, "build_library", lambda verbose=False: None)
+    monkeypatch.setattr(b, "build_host", lambda: made.append(1))
+    b.build()
+    assert not made  # up to date
+    monkeypatch.setattr(torch, "__version__", "0.0.0+other")
+    b.build()
+    assert made
+    # and the module of the other version is not loaded in its place
+    with pytest.raises(_cabi.FlagGemsB200Error, match="not found"):
+        _cabi._NativeHost().act_quant
