@@ -116,6 +116,9 @@ void fg_count_launch(int n);
 // global memory (it returns once every earlier kernel has finished and its writes are visible) and
 // fg_pdl_trigger() when the kernel after it may be scheduled.  What overlaps is launch latency and
 // prologues: ~2 us per kernel, which is a fifth of a decode-sized product.
+// Everything that an earlier kernel may have written, so any operand of a public entry point, is read with ordinary
+// loads.  The read-only path (__ldg, const __restrict__) is defined for memory that nobody writes while the kernel
+// lives, and that now includes the end of its predecessor; the compiler may also move such loads above the wait.
 __device__ __forceinline__ void fg_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void fg_pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -807,7 +807,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                     for (int c = 0; c < C::COLS / 32; ++c) {
                         const int n = min(out_col_base + 32 * (FUSE_SILU ? (c & 1) : c) + lane, p.n_out - 1);
                         const int up = FUSE_SILU && c >= 2 ? p.N / 2 : 0;
-                        s[c] = p.sb_mode == FG_SCALE_VECTOR ? __ldg(sbp + up + n) : __ldg(sbp);
+                        s[c] = p.sb_mode == FG_SCALE_VECTOR ? sbp[up + n] : sbp[0];
                         b[c] = p.bias ? load_as_float(p.bias, p.bias_dtype, n + (int64_t)expert * p.bias_stride_e) : 0.0f;
                     }
                     __syncwarp();  // every lane has read the previous tile's values
@@ -907,29 +907,26 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                 const bool as_vec = p.as_stride_k == 1 && ((reinterpret_cast<uintptr_t>(as_row) & 15) == 0);
                 const bool bs_vec = p.bs_stride_k == 1 && ((reinterpret_cast<uintptr_t>(bs0) & 15) == 0) &&
                                     ((reinterpret_cast<uintptr_t>(bs1) & 15) == 0);
-                auto load4 = [&](const float* base, int64_t stride, bool vec, int kb0, bool ldg) -> float4 {
-                    if (vec && (kb0 & 3) == 0 && kb0 + 4 <= num_k_blocks) {
-                        return ldg ? __ldg(reinterpret_cast<const float4*>(base + kb0))
-                                   : *reinterpret_cast<const float4*>(base + kb0);
-                    }
+                auto load4 = [&](const float* base, int64_t stride, bool vec, int kb0) -> float4 {
+                    if (vec && (kb0 & 3) == 0 && kb0 + 4 <= num_k_blocks) return *reinterpret_cast<const float4*>(base + kb0);
                     float v[4];
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const int kk = min(kb0 + i, num_k_blocks - 1);
-                        v[i] = ldg ? __ldg(base + (int64_t)kk * stride) : base[(int64_t)kk * stride];
+                        v[i] = base[(int64_t)kk * stride];
                     }
                     return make_float4(v[0], v[1], v[2], v[3]);
                 };
                 float4 a_nx = make_float4(0.f, 0.f, 0.f, 0.f), b0_nx = a_nx, b1_nx = a_nx;
                 float as_next = 0.f, b0_next = 0.f, b1_next = 0.f;
                 if constexpr (SCALE_GROUPS) {
-                    a_nx = load4(as_row, p.as_stride_k, as_vec, kb_begin, false);
-                    b0_nx = load4(bs0, p.bs_stride_k, bs_vec, kb_begin, true);
-                    b1_nx = FUSE_SILU ? load4(bs1, p.bs_stride_k, bs_vec, kb_begin, true) : b0_nx;
+                    a_nx = load4(as_row, p.as_stride_k, as_vec, kb_begin);
+                    b0_nx = load4(bs0, p.bs_stride_k, bs_vec, kb_begin);
+                    b1_nx = FUSE_SILU ? load4(bs1, p.bs_stride_k, bs_vec, kb_begin) : b0_nx;
                 } else {
                     as_next = as_row[(int64_t)kb_begin * p.as_stride_k];
-                    b0_next = __ldg(bs0 + (int64_t)kb_begin * p.bs_stride_k);
-                    if constexpr (FUSE_SILU) b1_next = __ldg(bs1 + (int64_t)kb_begin * p.bs_stride_k);
+                    b0_next = bs0[(int64_t)kb_begin * p.bs_stride_k];
+                    if constexpr (FUSE_SILU) b1_next = bs1[(int64_t)kb_begin * p.bs_stride_k];
                 }
                 float g0[4] = {0.f, 0.f, 0.f, 0.f}, g1[4] = {0.f, 0.f, 0.f, 0.f};  // products of the current group
                 for (int kb = kb_begin; kb < kb_end; ++kb) {
@@ -940,8 +937,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                         sc1f = FUSE_SILU ? as_next * b1_next : sc0f;
                         if (kb + 1 < kb_end) {  // next block's scales travel while this block is folded in
                             as_next = as_row[(int64_t)(kb + 1) * p.as_stride_k];
-                            b0_next = __ldg(bs0 + (int64_t)(kb + 1) * p.bs_stride_k);
-                            if constexpr (FUSE_SILU) b1_next = __ldg(bs1 + (int64_t)(kb + 1) * p.bs_stride_k);
+                            b0_next = bs0[(int64_t)(kb + 1) * p.bs_stride_k];
+                            if constexpr (FUSE_SILU) b1_next = bs1[(int64_t)(kb + 1) * p.bs_stride_k];
                         }
                     } else {
                         if (in_group == 0) {
@@ -950,9 +947,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                                 g1[0] = a_nx.x * b1_nx.x; g1[1] = a_nx.y * b1_nx.y; g1[2] = a_nx.z * b1_nx.z; g1[3] = a_nx.w * b1_nx.w;
                             }
                             if (kb + 4 < kb_end) {
-                                a_nx = load4(as_row, p.as_stride_k, as_vec, kb + 4, false);
-                                b0_nx = load4(bs0, p.bs_stride_k, bs_vec, kb + 4, true);
-                                if constexpr (FUSE_SILU) b1_nx = load4(bs1, p.bs_stride_k, bs_vec, kb + 4, true);
+                                a_nx = load4(as_row, p.as_stride_k, as_vec, kb + 4);
+                                b0_nx = load4(bs0, p.bs_stride_k, bs_vec, kb + 4);
+                                if constexpr (FUSE_SILU) b1_nx = load4(bs1, p.bs_stride_k, bs_vec, kb + 4);
                             }
                         }
                         sc0f = in_group == 0 ? g0[0] : in_group == 1 ? g0[1] : in_group == 2 ? g0[2] : g0[3];
@@ -1140,7 +1137,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const int n = min(n0 + c + i, p.n_out - 1);
-                        const float sb = p.sb_mode == FG_SCALE_VECTOR ? __ldg(p.sb + n) : p.sb[0];
+                        const float sb = p.sb_mode == FG_SCALE_VECTOR ? p.sb[n] : p.sb[0];
                         float x = sb * (sa * o[i]);
                         if (p.bias) {
                             const float b = load_as_float(p.bias, p.bias_dtype, n);

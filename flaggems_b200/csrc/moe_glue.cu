@@ -239,8 +239,8 @@ __global__ void __launch_bounds__(ALIGN_THREADS, 1) moe_align_kernel(AlignArgs a
 
 // ---------------------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(256) silu_and_mul_kernel(const T* __restrict__ x, const T* __restrict__ y,
-                                                           T* __restrict__ out, int64_t M, int64_t N, int64_t ld_x,
+__global__ void __launch_bounds__(256) silu_and_mul_kernel(const T* x, const T* y,
+                                                           T* out, int64_t M, int64_t N, int64_t ld_x,
                                                            int64_t ld_y, int64_t ld_o) {
     fg_pdl_wait();
     fg_pdl_trigger();
@@ -262,9 +262,9 @@ __global__ void __launch_bounds__(256) silu_and_mul_kernel(const T* __restrict__
 // slots' 16-byte loads are issued before the first add (HBM-bound: 1 GB per step of the
 // DeepSeek-V3 layer); TOPK == 0: any top-k, one load at a time.
 template <typename T, int TOPK>
-__global__ void __launch_bounds__(256) moe_sum_kernel(const T* __restrict__ in, T* __restrict__ out, int64_t M,
-                                                      int topk, int64_t K, const int32_t* __restrict__ row_index,
-                                                      const T* __restrict__ addend) {
+__global__ void __launch_bounds__(256) moe_sum_kernel(const T* in, T* out, int64_t M,
+                                                      int topk, int64_t K, const int32_t* row_index,
+                                                      const T* addend) {
     fg_pdl_wait();
     fg_pdl_trigger();
     const int64_t vec_per_row = K / 8;
@@ -327,13 +327,13 @@ __global__ void __launch_bounds__(256) moe_sum_kernel(const T* __restrict__ in, 
 // One warp per destination row, eight 16-byte loads per lane in flight before the first store
 // (measured 142 us against 148 with four, and 158 with plain instead of streaming stores, for the
 // 82688 rows of the DeepSeek-V3-shaped step: the destination is a 611 MB write stream).
-__global__ void __launch_bounds__(256) gather_rows_kernel(const uint8_t* __restrict__ src_q,
-                                                          const float* __restrict__ src_s, uint8_t* __restrict__ dst_q,
-                                                          float* __restrict__ dst_s, int64_t rows, int64_t K,
+__global__ void __launch_bounds__(256) gather_rows_kernel(const uint8_t* src_q,
+                                                          const float* src_s, uint8_t* dst_q,
+                                                          float* dst_s, int64_t rows, int64_t K,
                                                           int64_t s_cols, int64_t src_q_stride, int64_t src_s_stride,
-                                                          const int32_t* __restrict__ row_index,
+                                                          const int32_t* row_index,
                                                           int32_t index_div, int32_t index_limit,
-                                                          const int32_t* __restrict__ n_rows_dev) {
+                                                          const int32_t* n_rows_dev) {
     fg_pdl_wait();
     fg_pdl_trigger();
     if (n_rows_dev) {
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const uint8_t* __restr
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 const int v = v0 + 32 * u;
-                t[u] = (real && v < nvec) ? __ldg(sq + v) : make_uint4(0u, 0u, 0u, 0u);
+                t[u] = (real && v < nvec) ? sq[v] : make_uint4(0u, 0u, 0u, 0u);
             }
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
@@ -371,8 +371,8 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const uint8_t* __restr
 
 // Group of every row from the ends of the groups: ids[r] = number of offsets <= r (rows past the last
 // end get num_groups, which the alignment kernel ignores).
-__global__ void __launch_bounds__(256) group_ids_kernel(const int32_t* __restrict__ offs, int num_groups, int64_t rows,
-                                                        int32_t* __restrict__ ids) {
+__global__ void __launch_bounds__(256) group_ids_kernel(const int32_t* offs, int num_groups, int64_t rows,
+                                                        int32_t* ids) {
     fg_pdl_wait();
     fg_pdl_trigger();
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x) {
@@ -389,10 +389,10 @@ __global__ void __launch_bounds__(256) group_ids_kernel(const int32_t* __restric
 // The alignment tables of rows that are already grouped (group g = rows [offs[g-1], offs[g])): the same
 // sorted_ids / expert_ids / num_post_pad as moe_align on the rows' group ids, straight from the ends.
 // Every CTA scans the padded group sizes for itself and fills its share of sorted_ids.
-__global__ void __launch_bounds__(ALIGN_THREADS, 1) group_tiles_kernel(const int32_t* __restrict__ offs, int num_groups,
-                                                                       int32_t rows, int32_t block, int32_t* __restrict__ sorted_ids,
-                                                                       int64_t max_pad, int32_t* __restrict__ expert_ids,
-                                                                       int64_t n_blocks, int32_t* __restrict__ num_post_pad) {
+__global__ void __launch_bounds__(ALIGN_THREADS, 1) group_tiles_kernel(const int32_t* offs, int num_groups,
+                                                                       int32_t rows, int32_t block, int32_t* sorted_ids,
+                                                                       int64_t max_pad, int32_t* expert_ids,
+                                                                       int64_t n_blocks, int32_t* num_post_pad) {
     fg_pdl_wait();
     fg_pdl_trigger();
     __shared__ int32_t first[ALIGN_THREADS], pad_first[ALIGN_THREADS + 1], scan_tmp[ALIGN_WARPS];
@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(ALIGN_THREADS, 1) group_tiles_kernel(const int
     if (blockIdx.x == 0 && threadIdx.x == 0) num_post_pad[0] = total;
 }
 
-__global__ void __launch_bounds__(256) fill_ones_kernel(float* __restrict__ x, int64_t n) {
+__global__ void __launch_bounds__(256) fill_ones_kernel(float* x, int64_t n) {
     fg_pdl_wait();
     fg_pdl_trigger();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) x[i] = 1.0f;

@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(256, 5) group_quant16_kernel(QuantArgs a) {
 // payload, then its scales); this kernel copies the staged row of route slot order[r] to output row
 // r (a local packed buffer, or this rank's region of the destination rank's receive buffer) and
 // writes the row's trailer.  One warp per row, four 16-byte loads in flight per lane.
-__global__ void __launch_bounds__(256) pack_copy_kernel(QuantArgs a, const uint8_t* __restrict__ staged) {
+__global__ void __launch_bounds__(256) pack_copy_kernel(QuantArgs a, const uint8_t* staged) {
     fg_pdl_wait();
     fg_pdl_trigger();
     const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
@@ -584,10 +584,10 @@ int launch_rows(int dtype, const QuantArgs& a, cudaStream_t st) {
 // one atomicMax per block on the bit pattern (non-negative floats order like unsigned integers).
 // With row_index: over the rows that it names, entries outside [0, index_limit) skipped.
 template <typename T>
-__global__ void __launch_bounds__(256) abs_max_kernel(const T* __restrict__ x, int64_t rows, int64_t K, int64_t ld_x,
-                                                      const int32_t* __restrict__ n_rows_dev,
-                                                      const int32_t* __restrict__ row_index, int32_t index_limit,
-                                                      unsigned int* __restrict__ amax) {
+__global__ void __launch_bounds__(256) abs_max_kernel(const T* x, int64_t rows, int64_t K, int64_t ld_x,
+                                                      const int32_t* n_rows_dev,
+                                                      const int32_t* row_index, int32_t index_limit,
+                                                      unsigned int* amax) {
     fg_pdl_wait();
     fg_pdl_trigger();
     if (n_rows_dev) {
