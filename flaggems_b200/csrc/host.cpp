@@ -8,6 +8,8 @@
 // that called it goes through its checks, conversions and error messages.
 #include <Python.h>
 
+#include <algorithm>
+
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -537,14 +539,14 @@ PyObject* fused_experts(PyObject*, PyObject* const* p, Py_ssize_t n) {
         const at::Tensor* map = nullptr;
         if (p[12] != Py_None && !(map = cuda_tensor(p[12]))) return none();
         const int64_t t = x->size(0), h = x->size(1), inter = w2->size(2), topk = ids->size(1);
-        if (experts < w1->size(0)) experts = w1->size(0);  // more weights than the count names: ids stay below it
         const int code = dtype_code(x->scalar_type()), esz = (int)x->element_size();
         const bool i64 = ids->scalar_type() == ScalarType::Long;
         at::Tensor ws;
         const int rc = unlocked([&] {
             c10::cuda::CUDAGuard guard(x->device());
             const int64_t most = t < chunk ? t : chunk;
-            const int64_t need = fg_fused_experts_workspace_bytes((int)mode, most, (int)topk, (int)experts, h, inter, code);
+            const int64_t need = fg_fused_experts_workspace_bytes(
+                (int)mode, most, (int)topk, (int)std::max(experts, w1->size(0)), h, inter, code);
             ws = empty({need}, ScalarType::Byte, *x);
             for (int64_t b = 0; b < t; b += chunk) {
                 const int64_t rows = t - b < chunk ? t - b : chunk;

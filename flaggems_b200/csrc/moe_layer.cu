@@ -380,7 +380,7 @@ int fg_moe_routed_block_fp8_local_noalloc(void* y, const void* hidden, int hidde
                                          w1, w2, s1, s2, num_experts, H, I, scratch, FG_NOALLOC_SCRATCH_BYTES, stream);
 }
 
-// Workspace of fg_fused_experts in one mode.
+// Workspace of fg_fused_experts in one mode.  num_experts: the larger of the ids' range and the number of weights.
 static Workspace carve_experts(void* base, int mode, int64_t T, int topk, int num_experts, int64_t H, int64_t I, int esz) {
     Workspace w{};
     Carver c{reinterpret_cast<uint8_t*>(base), 0};
@@ -418,17 +418,17 @@ int fg_fused_experts(void* out, const void* hidden, int hidden_dtype, const void
     FG_REQUIRE(out && hidden && topk_ids && topk_w && w1 && w2 && workspace && (mode == FG_EXPERTS_16BIT || (s1 && s2)),
                FG_ERR_INVALID_ARGUMENT, "null pointer");
     FG_REQUIRE(T * topk < (1ll << 31), FG_ERR_UNSUPPORTED, "too many route slots");
-    FG_REQUIRE(local_experts <= num_experts, FG_ERR_INVALID_ARGUMENT, "more local experts than experts");
-    const Workspace ws = carve_experts(workspace, mode, T, topk, num_experts, H, I, hidden_dtype == FG_DTYPE_F32 ? 4 : 2);
+    const int widest = num_experts > local_experts ? num_experts : local_experts;
+    const Workspace ws = carve_experts(workspace, mode, T, topk, widest, H, I, hidden_dtype == FG_DTYPE_F32 ? 4 : 2);
     FG_REQUIRE((uintptr_t)workspace % 256 == 0 && workspace_bytes >= ws.bytes, FG_ERR_INVALID_ARGUMENT,
                "workspace holds %lld bytes, needs %lld (256-byte aligned)", (long long)workspace_bytes, (long long)ws.bytes);
-    const bool pairs = mode != FG_EXPERTS_BLOCK_FP8 && use_pairs(T * topk, num_experts, 2 * I, H);
+    const bool pairs = mode != FG_EXPERTS_BLOCK_FP8 && use_pairs(T * topk, widest, 2 * I, H);
     int rc = fg_moe_align(topk_ids, ids_are_i64, T * topk, num_experts, pairs ? PAIR_ROWS : TILE_ROWS, expert_map, expert_map_len, ws.sorted_ids,
                           ws.max_pad, ws.expert_ids, ws.n_blocks, ws.post_pad, 1, 1, nullptr, nullptr, 0, nullptr, 0, false,
                           (cudaStream_t)stream);
     if (rc != FG_OK) return rc;
     const Experts e{mode, hidden, hidden_dtype, topk_w, topk_w_dtype, T, topk, w1, w2, s1, s2, a1_scale, a2_scale,
-                    local_experts, H, I, use_gather(T * topk, num_experts), pairs};
+                    local_experts, H, I, use_gather(T * topk, widest), pairs};
     rc = run_experts(e, ws, ws.routed, (cudaStream_t)stream);
     if (rc != FG_OK) return rc;
     return fg_moe_sum_indexed(ws.routed, out, T, topk, H, hidden_dtype, nullptr, addend, stream);

@@ -266,8 +266,10 @@ int fg_moe_routed_block_fp8_local(void* y, const void* hidden, int hidden_dtype,
  *   FG_EXPERTS_TENSOR_FP8   e4m3, scales [E]; activations by a1_scale / a2_scale[0], or dynamic when NULL
  *   FG_EXPERTS_16BIT        bf16 / fp16 weights of hidden_dtype, no scales
  *   FG_EXPERTS_16BIT_SCALED the same with scales [E, 2I] and [E, H] on the accumulators
- * expert_map as in fg_moe_align_block_size (experts mapped to -1 contribute zeros).  Scratch is the
- * caller's workspace (256-byte aligned, fg_fused_experts_workspace_bytes). */
+ * topk_ids run over num_experts (slots with other ids have no row); w1 / w2 hold local_experts, which may be
+ * more or fewer.  expert_map as in fg_moe_align_block_size (experts mapped to -1 contribute zeros).
+ * Scratch is the caller's workspace (256-byte aligned, fg_fused_experts_workspace_bytes for the larger of
+ * the two counts). */
 #define FG_EXPERTS_BLOCK_FP8 0
 #define FG_EXPERTS_CHANNEL_FP8 1
 #define FG_EXPERTS_CHANNEL_INT8 2

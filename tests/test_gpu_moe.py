@@ -107,6 +107,36 @@ def test_fused_moe_per_tensor_ignores_unrouted_slots():
     assert torch.equal(out[1:], ref)
 
 
+def test_fused_moe_fewer_experts_than_weights():
+    # ids run over the first `global_num_experts`; the other weights are there but nothing selects them
+    g = torch.Generator().manual_seed(6)
+    t, h, i, e, topk = 21, 256, 256, 6, 2
+    hidden = torch.randn(t, h, generator=g).bfloat16()
+    w1 = (torch.randn(e, 2 * i, h, generator=g) * 20).clamp(-448, 448).to(FP8).cuda()
+    w2 = (torch.randn(e, h, i, generator=g) * 20).clamp(-448, 448).to(FP8).cuda()
+    s1, s2 = torch.full((e,), 1e-3, device="cuda"), torch.full((e,), 1e-3, device="cuda")
+    s1[5] = 0.1  # would set the scale of the intermediate rows
+    tw, ti = _router(t, 4, topk, g)
+
+    def run(x, ids, w, n, **how):
+        return flag_gems.fused_experts_impl(x.cuda(), w1[:n], w2[:n], w.cuda(), ids.cuda(), use_fp8_w8a8=True, w1_scale=s1[:n],
+                                            w2_scale=s2[:n], **how)
+
+    def table(*entries):
+        return torch.tensor(entries, dtype=torch.int32, device="cuda")
+
+    # an expert map shorter than the weights, one of its experts elsewhere
+    ref = run(hidden, torch.tensor([2, 3, 4, 0])[ti.long()], tw, 6, expert_map=table(0, 1, 2, 3, -1, 5))
+    out = run(hidden, ti, tw, 6, global_num_experts=4, expert_map=table(2, 3, -1, 0))
+    assert torch.equal(out, ref) and out.abs().max() > 0
+    # ids at and above the count have no row, although there are weights for them
+    ref = run(hidden[1:], ti[1:], tw[1:], 4)
+    hidden[0] = hidden[1]
+    ti[0] = 5
+    out = run(hidden, ti, tw, 6, global_num_experts=4)
+    assert torch.equal(out[1:], ref)
+
+
 @pytest.mark.parametrize("block_m", [16, 64, 128])
 @pytest.mark.parametrize("mode", ["block", "channel", "tensor"])
 def test_dispatch_fused_moe_kernel(block_m, mode):
