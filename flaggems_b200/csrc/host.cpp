@@ -59,6 +59,14 @@ bool py_int(PyObject* o, int64_t* out) {
     return true;
 }
 
+// Truth of a Python object; false where it has none (the Python code then raises what asking for it raises).
+bool py_bool(PyObject* o, bool* out) {
+    const int v = PyObject_IsTrue(o);
+    if (v < 0) PyErr_Clear();
+    *out = v == 1;
+    return v >= 0;
+}
+
 at::Tensor empty(at::IntArrayRef sizes, ScalarType dtype, const at::Tensor& like) {
     return at::Tensor(at::detail::empty_cuda(sizes, dtype, like.device(), std::nullopt));
 }
@@ -160,8 +168,8 @@ PyObject* group_quant(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (n != 5 || !PyFloat_Check(a[2]) || !py_int(a[1], &group) || group <= 0) return none();
         const at::Tensor* x = cuda_tensor(a[0]);
         if (!x || dtype_code(x->scalar_type()) < 0 || !as_rows(*x, &m, &k, &ld) || k % group) return none();
-        const bool column = PyObject_IsTrue(a[3]) == 1, ue8m0 = PyObject_IsTrue(a[4]) == 1;
-        if (column && x->dim() != 2) return none();
+        bool column, ue8m0;
+        if (!py_bool(a[3], &column) || !py_bool(a[4], &ue8m0) || (column && x->dim() != 2)) return none();
         const float eps = (float)PyFloat_AS_DOUBLE(a[2]);
         const int64_t g = k / group;
         at::Tensor q, s;
@@ -187,7 +195,8 @@ PyObject* act_quant(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const at::Tensor* x = cuda_tensor(a[0]);
         if (!x || x->scalar_type() != ScalarType::BFloat16 || !x->is_contiguous() || !as_rows(*x, &m, &k, &ld) || k % block)
             return none();
-        const bool pow2 = PyObject_IsTrue(a[2]) == 1;
+        bool pow2;
+        if (!py_bool(a[2], &pow2)) return none();
         at::Tensor y, s;
         const int rc = unlocked([&] {
             c10::cuda::CUDAGuard guard(x->device());
@@ -305,7 +314,7 @@ PyObject* scaled_mm(PyObject*, PyObject* const* p, Py_ssize_t n) {
         if (code < 0 || m == 0 || cols == 0 || b->size(0) != k || c->size(0) != m || c->size(1) != cols) return none();
         if (a->stride(1) != 1 || a->stride(0) % 16 || c->stride(1) != 1 || !k_contiguous(*b)) return none();
         if (!scale_ok(*sa, m) || !scale_ok(*sb, cols)) return none();
-        const bool cutlass = PyObject_IsTrue(p[6]) == 1;
+        const bool cutlass = p[6] == Py_True;
         if (cutlass) {
             if (c->stride(0) % 16 || code == FG_DTYPE_E4M3) return none();
         } else {
@@ -395,7 +404,8 @@ PyObject* topk_softmax(PyObject*, PyObject* const* p, Py_ssize_t n) {
         const ScalarType it = idx->scalar_type();
         const int kind = it == ScalarType::Int ? 0 : it == ScalarType::UInt32 ? 1 : it == ScalarType::Long ? 2 : -1;
         if (kind < 0 || dtype_code(g->scalar_type()) < 0) return none();
-        const bool renormalize = PyObject_IsTrue(p[4]) == 1;
+        bool renormalize;
+        if (!py_bool(p[4], &renormalize)) return none();
         const int rc = unlocked([&] {
             c10::cuda::CUDAGuard guard(g->device());
             return fg_topk_softmax(static_cast<float*>(w->data_ptr()), idx->data_ptr(), kind, static_cast<int32_t*>(src->data_ptr()),
@@ -420,7 +430,8 @@ PyObject* grouped_topk(PyObject*, PyObject* const* p, Py_ssize_t n) {
         if (t == 0 || n_group < 1 || n_group > 32 || e % n_group || topk > 32 || (scoring != 0 && scoring != 1)) return none();
         if (s->stride(1) != 1 || bias->scalar_type() != s->scalar_type() || bias->size(0) != e || !bias->is_contiguous())
             return none();
-        const bool renormalize = PyObject_IsTrue(p[4]) == 1;
+        bool renormalize;
+        if (!py_bool(p[4], &renormalize)) return none();
         const float scaling = (float)PyFloat_AS_DOUBLE(p[5]);
         at::Tensor w, idx;
         const int rc = unlocked([&] {

@@ -129,3 +129,14 @@ def test_other_threads_run_while_a_call_blocks():
     torch.cuda.synchronize()
     assert blocked > 0.3, "the launch queue never filled: nothing was tested"
     assert max(b - a for a, b in zip(ticks, ticks[1:])) < 0.15
+
+
+def test_a_flag_without_a_truth_value_raises_its_own_error():
+    both = torch.ones(2, dtype=torch.bool)
+    x = _rand(9, 256)
+    for call in (lambda: flag_gems.per_token_group_quant_fp8(x, 128, scale_ue8m0=both),
+                 lambda: flag_gems.per_token_group_quant_fp8(x, 128, column_major_scales=both),
+                 lambda: flag_gems.grouped_topk(x, 4, 2, 4, both, 2.5, x[0], 1),
+                 lambda: flag_gems.topk_softmax(*_topk(torch.int32), x[:5, :16].contiguous(), both)):
+        with pytest.raises(RuntimeError, match="ambiguous"):
+            call()
