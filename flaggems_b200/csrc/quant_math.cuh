@@ -1,5 +1,5 @@
-// Arithmetic of the quantisation rules, shared by the quantisation kernels and the GEMM epilogue that
-// quantises its output.  All of it is IEEE fp32: the same inputs give the same bits wherever it runs.
+// Arithmetic of the quantisation rules, for the kernels of quant.cu.  All of it is IEEE fp32: the same inputs give
+// the same bits in each of them.
 #pragma once
 #include "common.cuh"
 

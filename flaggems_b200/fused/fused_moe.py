@@ -4,14 +4,14 @@ quantise -> grouped GEMM2 (x router weight) -> top-k sum.
 Mirrors the FP8 path of src/flag_gems/fused/fused_moe.py of the reference:
 ``fused_experts_impl`` (:1821-2185), ``inplace_fused_experts`` / ``outplace_fused_experts``
 (:2188-2290), ``_fp8_quantize`` / ``moe_kernel_quantize_input`` (:629-698, :749-773),
-``MoEActivation`` (:538-577).  The two grouped GEMMs are ``fg_moe_grouped_gemm_fp8``
-(tcgen05); a layer runs as one native call (``fg_fused_experts``), whose GEMMs fetch their rows
-through ``sorted_ids``.
+``MoEActivation`` (:538-577).  A layer runs as one native call (``fg_fused_experts``) on the grouped
+tcgen05 GEMM: with few rows per expert its products fetch their rows through ``sorted_ids``, otherwise the
+rows are laid out in expert order first.
 
-Implemented: the FP8 w8a8 modes (block 128x128, per-token x per-channel, per-tensor) and int8
-w8a8 with per-token x per-channel scales (tcgen05 kind::i8, int32 accumulation); the weight-only
-(w8a16 / w4a16), MX, bias and non-SiLU options of the reference signature raise
-NotImplementedError.
+Implemented: the FP8 w8a8 modes (block 128x128, per-token x per-channel, per-tensor), int8 w8a8 with
+per-token x per-channel scales (tcgen05 kind::i8, int32 accumulation), unquantised 16-bit experts and the
+weight-only forms (int8 / int4 in int8 containers); the MX, zero-point, bias and non-SiLU options of the
+reference signature raise NotImplementedError.
 """
 import logging
 from enum import Enum

@@ -10,8 +10,8 @@ and error messages (:262-366), same four operand forms:
 
 with ``out = ((A @ B) * scale_a[:, None]) * scale_b[None, :] (+ bias in fp32)`` cast to ``out_dtype``
 (bf16 by default for FP8 inputs).  The first form is the device primitive
-(``fg_scaled_grouped_mm_fp8``: group ids from the offsets, alignment to 128-row tiles, row gather,
-grouped tcgen05 GEMM with the rows scattered back; ``offs`` is read on the device).  The other
+(``fg_scaled_grouped_mm_fp8``: tile tables straight from the offsets, then the grouped tcgen05 GEMM, which reads
+the rows where they lie and writes them back there; ``offs`` is read on the device).  The other
 three are expressed through it here: the batched form as one grouped product over the flattened
 rows, the B-2-D form as the transposed problem, the K-split form as products of A with everything
 outside a group's K range zeroed.

@@ -247,8 +247,9 @@ int fg_ep_pack_rows_fp8_peer(const void* x, int x_dtype, int64_t T, int64_t K, i
 int64_t fg_moe_routed_workspace_bytes(int64_t n_rows_in, int num_experts, int64_t H, int64_t I);
 
 /* All experts local: y[T*topk, H] (route-slot order) = w2[e] . quant(silu_mul(w1[e] . quant(x)))
- * times the router weight, for every (token, slot).  Five launches (align, quantise, GEMM1+SiLU
- * on gathered rows, quantise, GEMM2), no allocation: scratch is the caller's workspace (256-byte
+ * times the router weight, for every (token, slot).  Five launches (align, quantise, GEMM1+SiLU,
+ * quantise, GEMM2): with few rows per expert the GEMMs gather their rows, otherwise rows are laid out in
+ * expert order, by a sixth launch when topk > 2.  No allocation: scratch is the caller's workspace (256-byte
  * aligned, fg_moe_routed_workspace_bytes(T*topk, ...)). */
 int fg_moe_routed_block_fp8_local(void* y, const void* hidden, int hidden_dtype, const void* topk_ids,
                                   int ids_are_i64, const void* topk_w, int topk_w_dtype, int64_t T,
