@@ -418,6 +418,9 @@ int fg_fused_experts(void* out, const void* hidden, int hidden_dtype, const void
     FG_REQUIRE(out && hidden && topk_ids && topk_w && w1 && w2 && workspace && (mode == FG_EXPERTS_16BIT || (s1 && s2)),
                FG_ERR_INVALID_ARGUMENT, "null pointer");
     FG_REQUIRE(T * topk < (1ll << 31), FG_ERR_UNSUPPORTED, "too many route slots");
+    // Gathered 16-bit rows are read where they lie; the other orders check their rows when they copy or quantise them.
+    FG_REQUIRE(mode < FG_EXPERTS_16BIT || ((uintptr_t)hidden % 16 == 0 && H % 8 == 0), FG_ERR_UNSUPPORTED,
+               "hidden rows must be 16-byte aligned (ptr %p, %lld elements)", hidden, (long long)H);
     const int widest = num_experts > local_experts ? num_experts : local_experts;
     const Workspace ws = carve_experts(workspace, mode, T, topk, widest, H, I, hidden_dtype == FG_DTYPE_F32 ? 4 : 2);
     FG_REQUIRE((uintptr_t)workspace % 256 == 0 && workspace_bytes >= ws.bytes, FG_ERR_INVALID_ARGUMENT,

@@ -464,3 +464,13 @@ def test_fused_moe_cta_pairs_match_single_ctas(mode):
                      for b in range(0, t, 100)])
     assert torch.isfinite(out).all() and out.float().abs().max() > 0
     assert torch.equal(out, ref)
+
+
+@pytest.mark.parametrize("tokens", [2, 200])  # rows gathered by the products, rows copied into expert order
+@pytest.mark.parametrize("mode", ["channel", "bf16"])
+def test_fused_moe_refuses_misaligned_rows(mode, tokens):
+    w1, w2, how = _wide_experts(mode, 2, 128, 128, torch.Generator(device="cuda").manual_seed(1))
+    hidden = torch.zeros(tokens * 128 + 1, dtype=torch.bfloat16, device="cuda")[1:].view(tokens, 128)
+    tw, ti = torch.ones(tokens, 1, device="cuda"), torch.zeros(tokens, 1, dtype=torch.int32, device="cuda")
+    with pytest.raises(NotImplementedError, match="16-byte aligned"):
+        flag_gems.fused_experts_impl(hidden, w1, w2, tw, ti, **how)
