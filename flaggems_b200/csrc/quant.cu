@@ -512,14 +512,14 @@ __global__ void __launch_bounds__(1024) row_quant16_kernel(QuantArgs a) {
     const int64_t src = source_row(a, row);
     const int units = (int)(a.K / 16);
     uint4* q = reinterpret_cast<uint4*>(a.q + row * a.ld_q);
-    float s;
-    if constexpr (MODE == QM_TENSOR_STATIC) {
-        s = a.tensor_scale[0];
-    } else if constexpr (MODE == QM_TENSOR_DYNAMIC) {
-        s = __fdiv_rn(fmaxf(a.tensor_scale[0], __uint_as_float(0x2edbe6ffu)), 448.0f);
-        if (row == 0 && threadIdx.x == 0) a.tensor_scale_out[0] = s;  // row 0 may be a padding row
-    }
+    // the one scale of a dynamic tensor: row 0 writes it, a padding row or not
+    auto dynamic_scale = [&]() -> float {
+        const float s = __fdiv_rn(fmaxf(a.tensor_scale[0], __uint_as_float(0x2edbe6ffu)), 448.0f);
+        if (row == 0 && threadIdx.x == 0) a.tensor_scale_out[0] = s;
+        return s;
+    };
     if (src < 0) {  // padding row
+        if constexpr (MODE == QM_TENSOR_DYNAMIC) dynamic_scale();
         for (int u = threadIdx.x; u < units; u += blockDim.x) q[u] = make_uint4(0u, 0u, 0u, 0u);
         if (!TENSOR && threadIdx.x == 0) a.s[row * a.s_row_stride] = make_scale<MODE>(0.0f, a.eps, a.pow2);
         return;
@@ -532,7 +532,12 @@ __global__ void __launch_bounds__(1024) row_quant16_kernel(QuantArgs a) {
         v[j][0] = u < units ? x[2 * u] : make_uint4(0u, 0u, 0u, 0u);
         v[j][1] = u < units ? x[2 * u + 1] : make_uint4(0u, 0u, 0u, 0u);
     }
-    if constexpr (!TENSOR) {
+    float s;  // after the row's loads: a division in front of them holds them back
+    if constexpr (MODE == QM_TENSOR_STATIC) {
+        s = a.tensor_scale[0];
+    } else if constexpr (MODE == QM_TENSOR_DYNAMIC) {
+        s = dynamic_scale();
+    } else {
         typename P::V m2 = typename P::V();
 #pragma unroll
         for (int j = 0; j < ROW_UNITS; ++j) m2 = absmax16<T>(m2, v[j]);
